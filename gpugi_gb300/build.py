@@ -35,7 +35,7 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contra
 NVCC_FLAGS += os.environ.get("GPUGI_NVCC_EXTRA", "").split()
 
 CUDA_SOURCES = ["trace.cu", "scene.cu", "render.cu", "capi.cu", "host.cu", "noalloc.cu", "nrc.cu", "tune.cu", "build.cu",
-                "hierarchy.cu"]
+                "hierarchy.cu", "wide.cu"]
 
 
 def _run(cmd):

@@ -589,6 +589,7 @@ static gpugi_status build_into(gpugi_ctx* ctx, gpugi_scene* sc, const float* pos
     sc->dev.numMaterials = numMaterials;
     sc->dev.topNodes = 0;
     sc->numLeafBlocks = numBlocks;
+    if ((gs = build_wide(ctx, sc))) return gs;
     // Host copies for the light tables (Scene::LoadLightSources): only the
     // emissive triangles, in input order, each with its own three vertices.
     bool anyEmissive = false;

@@ -22,7 +22,7 @@ struct gpugi_ctx {
     void* stageDev = nullptr;
     size_t stageDevBytes = 0;
     // trace tuning
-    uint32_t traceMode = 3;  // 0 thread per ray, 1 persistent lane refill, 2 root prefilter + 1, 3/4 + 8/4-lane groups
+    uint32_t traceMode = 3;  // 0 thread per ray, 1 persistent lane refill, 2 root prefilter + 1, 3 + wide walk or 8-lane groups, 4/5 + 4/16-lane groups
     uint32_t traceBlock = 128;
     // photon mapper (PhotonMapper's pm_nphotons, pm_r, pm_progressive; photonmapper.cpp:17-45)
     uint32_t pmPhotonsPerSample = 1u << 11;
@@ -101,6 +101,7 @@ struct gpugi_scene {
     std::vector<int32_t> hostSlots;
     std::vector<float> hostMaterials;
     uint32_t numLeafBlocks = 0;
+    const float4* wide = nullptr;  // dev.wide before gpugi_debug_limit_nodes
     uint32_t numNodesUploaded = 0;  // dev.numNodes before gpugi_debug_limit_nodes
     // light tables (Scene::LoadLightSources / ComputePointLightTable)
     bool lightsReady = false;
@@ -200,6 +201,9 @@ gpugi_status nrc_train_counted(gpugi_ctx* ctx, gpugi_nrc* nn, const float* sampl
 // Per-slot triangle records {p0, e0, e1, n} of a device slot array (scene.cu).
 void prepare_triangles(cudaStream_t stream, const int4* slots, uint32_t numSlots, const float* positions,
                        float4* tris);
+// Derives the scene's four-wide hierarchy from its binary one on the device, where the tree
+// allows it (wide.cu); leaves dev.wide null otherwise.
+gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc);
 // Light tables and the host light sampler (host.cu).
 void build_light_tables(gpugi_scene* sc);
 void generate_light_samples(gpugi_scene* sc, uint64_t& rng, uint32_t numSamples, float* out);

@@ -265,10 +265,48 @@ __global__ void __launch_bounds__(128) k_shadow(RenderConst rc, ShadowSoA Q, int
     }
 }
 
+// The same queues on scenes with a wide hierarchy (wide_walks).
+__global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_extend_wide(RenderConst rc, PathSoA A, HitSoA H,
+                                                                            int depth) {
+    __shared__ WideShared sh;
+    const uint32_t n = rc.cnt->path[depth];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&rc.cnt->rays[0], (unsigned long long)n);
+    wide_walks<false, 0>(
+        sh, rc.s, n, &rc.cnt->extendWork[depth], rc.err,
+        [&](uint32_t i, float3& o, float3& d, float& tmax) {
+            o = make_float3(A.ox[i], A.oy[i], A.oz[i]);
+            d = make_float3(A.dx[i], A.dy[i], A.dz[i]);
+            tmax = kRAY_MAX;
+        },
+        [&](uint32_t i, int32_t slot, float t, float u, float v) {
+            H.slot[i] = slot;
+            H.t[i] = t;
+            H.u[i] = u;
+            H.v[i] = v;
+        });
+}
+
+__global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_shadow_wide(RenderConst rc, ShadowSoA Q, int depth) {
+    __shared__ WideShared sh;
+    const uint32_t n = rc.cnt->shadow[depth];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&rc.cnt->rays[1], (unsigned long long)n);
+    wide_walks<true, 0>(
+        sh, rc.s, n, &rc.cnt->shadowWork[depth], rc.err,
+        [&](uint32_t i, float3& o, float3& d, float& tmax) {
+            o = make_float3(Q.ox[i], Q.oy[i], Q.oz[i]);
+            d = make_float3(Q.dx[i], Q.dy[i], Q.dz[i]);
+            tmax = Q.tmax[i];
+        },
+        [&](uint32_t i, int32_t slot, float, float, float) {
+            if (slot < 0) shadow_unoccluded(rc, Q, i);
+        });
+}
+
 // Launch shapes and launches of the walkers for a scene: group walks when the
 // context's trace mode is 3 or 4, else lane walks with staged top nodes.
 struct Walkers {
     int bounds = 0;  // node kind: 0 box, 1 ellipsoid, 2 oriented box
+    bool wide = false;  // walks on the wide hierarchy
     uint32_t groupBelowE = 0, groupBelowS = 0;  // queue lengths below which groups walk
     WalkerLaunch LE, LS;
 };
@@ -2062,6 +2100,11 @@ static gpugi_status ensure_buffers_in(gpugi_ctx* ctx, RenderBuffers* rb, size_t 
 
 static gpugi_status walkers_config(gpugi_ctx* ctx, const gpugi_scene* sc, Walkers& W) {
     W.bounds = (int)sc->dev.boundsKind;
+    W.wide = sc->dev.wide && ctx->traceMode == 3;
+    if (W.wide) {
+        gpugi_status st = walker_launch_config(ctx, sc, (const void*)k_extend_wide, 1ull << 40, 0, W.LE);
+        return st ? st : walker_launch_config(ctx, sc, (const void*)k_shadow_wide, 1ull << 40, 0, W.LS);
+    }
     const void* ke = W.bounds == 1 ? (const void*)k_extend<1>
                      : W.bounds == 2 ? (const void*)k_extend<2> : (const void*)k_extend<0>;
     const void* ks = W.bounds == 1 ? (const void*)k_shadow<1>
@@ -2081,14 +2124,16 @@ static gpugi_status walkers_config(gpugi_ctx* ctx, const gpugi_scene* sc, Walker
 static void launch_extend(gpugi_ctx* ctx, const Walkers& W, const RenderConst& rc, const PathSoA& A, const HitSoA& H,
                           int depth) {
     const WalkerLaunch& L = W.LE;
-    if (W.bounds == 1) k_extend<1><<<L.grid, 128, L.smem, ctx->stream>>>(rc, A, H, depth, L.stage, W.groupBelowE);
+    if (W.wide) k_extend_wide<<<L.grid, 128, 0, ctx->stream>>>(rc, A, H, depth);
+    else if (W.bounds == 1) k_extend<1><<<L.grid, 128, L.smem, ctx->stream>>>(rc, A, H, depth, L.stage, W.groupBelowE);
     else if (W.bounds == 2) k_extend<2><<<L.grid, 128, L.smem, ctx->stream>>>(rc, A, H, depth, L.stage, W.groupBelowE);
     else k_extend<0><<<L.grid, 128, L.smem, ctx->stream>>>(rc, A, H, depth, L.stage, W.groupBelowE);
 }
 
 static void launch_shadow(gpugi_ctx* ctx, const Walkers& W, const RenderConst& rc, const ShadowSoA& Q, int depth) {
     const WalkerLaunch& L = W.LS;
-    if (W.bounds == 1) k_shadow<1><<<L.grid, 128, L.smem, ctx->stream>>>(rc, Q, depth, L.stage, W.groupBelowS);
+    if (W.wide) k_shadow_wide<<<L.grid, 128, 0, ctx->stream>>>(rc, Q, depth);
+    else if (W.bounds == 1) k_shadow<1><<<L.grid, 128, L.smem, ctx->stream>>>(rc, Q, depth, L.stage, W.groupBelowS);
     else if (W.bounds == 2) k_shadow<2><<<L.grid, 128, L.smem, ctx->stream>>>(rc, Q, depth, L.stage, W.groupBelowS);
     else k_shadow<0><<<L.grid, 128, L.smem, ctx->stream>>>(rc, Q, depth, L.stage, W.groupBelowS);
 }

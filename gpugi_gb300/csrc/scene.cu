@@ -240,7 +240,6 @@ extern "C" gpugi_status gpugi_scene_upload(gpugi_ctx* ctx, const float* hierarch
     k_prepare_triangles<<<(numSlots + 255) / 256, 256, 0, ctx->stream>>>(dSlots, numSlots, dPos,
                                                                          const_cast<float4*>(dTris));
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "scene upload"));
 
     sc->dev.nodes = dNodes;
@@ -258,6 +257,8 @@ extern "C" gpugi_status gpugi_scene_upload(gpugi_ctx* ctx, const float* hierarch
     sc->dev.numVertices = numVertices;
     sc->dev.numMaterials = numMaterials;
     sc->dev.topNodes = topNodes;
+    if ((st = build_wide(ctx, sc))) return cleanup(st);
+    if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cleanup(cuda_fail(ctx, e, "scene upload"));
     sc->nodeMap.swap(nodeMap);
     sc->hostRadii.swap(hostRadii);
     sc->hostPositions.assign(positions, positions + 3 * (size_t)numVertices);
@@ -356,5 +357,7 @@ extern "C" gpugi_status gpugi_debug_limit_nodes(gpugi_scene* sc, uint32_t numNod
     if (numNodes > sc->numNodesUploaded)
         return fail(sc->ctx, GPUGI_ERROR_INVALID_ARGUMENT, "the node limit can only be lowered");
     sc->dev.numNodes = numNodes ? numNodes : sc->numNodesUploaded;
+    // the wide copy holds every node: a lowered limit is walked on the binary tree
+    sc->dev.wide = sc->dev.numNodes == sc->numNodesUploaded ? sc->wide : nullptr;
     return GPUGI_OK;
 }

@@ -25,6 +25,10 @@ struct DevScene {
     // watertight test records {p0.xyz p1.x | p1.yz p2.xy | p2.z 0 0 0} per leaf
     // slot, made on demand (gpugi_scene_set_triangle_test); null otherwise
     const float4* wtris = nullptr;
+    // four-wide copy of the hierarchy for the ray walkers (wide.cu), 8 float4
+    // per node; null where the binary tree does not allow it
+    const float4* wide = nullptr;
+    uint32_t numWide = 0;
     const int4* slots = nullptr;
     const float* positions = nullptr;
     const float4* vinfo = nullptr;

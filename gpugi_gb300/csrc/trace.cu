@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(128) k_trace_queue(
     }
 }
 
-// Group walker (modes 3 and 4), second launch after the root prefilter: G
+// Group walker (modes 4 and 5, and mode 3 on scenes without a wide hierarchy),
+// second launch after the root prefilter: G
 // lanes walk each queued ray together (group_step), which shortens the
 // dependent fetch chain of the longest walks.
 template <bool ANY_HIT, int BOUNDS, int G, int TRI>
@@ -344,6 +345,37 @@ __global__ void __launch_bounds__(128, GPUGI_GROUP_MIN_BLOCKS) k_trace_group(
                 t[ray] = g.len;
                 u[ray] = g.u;
                 v[ray] = g.v;
+            }
+        });
+}
+
+// Second launch after the root prefilter on scenes with a wide hierarchy: one
+// lane walks each queued ray over it (wide_walks).
+template <bool ANY_HIT, int TRI>
+__global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide(
+    DevScene s, const float* __restrict__ ox, const float* __restrict__ oy, const float* __restrict__ oz,
+    const float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ dz,
+    const float* __restrict__ tmax, int32_t* __restrict__ slot, float* __restrict__ t, float* __restrict__ u,
+    float* __restrict__ v, uint8_t* __restrict__ occluded, const uint32_t* __restrict__ queue,
+    unsigned long long* counters, uint32_t* err) {
+    __shared__ WideShared sh;
+    wide_walks<ANY_HIT, TRI>(
+        sh, s, counters[1], counters + 2, err,
+        [&](uint64_t i, float3& o, float3& d, float& len) {
+            const uint32_t ray = __ldg(queue + i);
+            o = make_float3(__ldg(ox + ray), __ldg(oy + ray), __ldg(oz + ray));
+            d = make_float3(__ldg(dx + ray), __ldg(dy + ray), __ldg(dz + ray));
+            len = __ldg(tmax + ray);
+        },
+        [&](uint64_t i, int32_t hitSlot, float hitT, float hitU, float hitV) {
+            const uint32_t ray = __ldg(queue + i);
+            if (ANY_HIT) {
+                occluded[ray] = hitSlot >= 0 ? 1 : 0;
+            } else {
+                slot[ray] = hitSlot;
+                t[ray] = hitT;
+                u[ray] = hitU;
+                v[ray] = hitV;
             }
         });
 }
@@ -407,6 +439,21 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
                                   slot ? slot + head : nullptr, t ? t + head : nullptr, u ? u + head : nullptr,
                                   v ? v + head : nullptr, occluded ? occluded + head : nullptr, queue, counters,
                                   (uint32_t)head);
+    }
+    if (ctx->traceMode == 3 && sc->dev.wide) {
+        auto kw = anyHit ? (wt ? &k_trace_wide<true, 1> : &k_trace_wide<true, 0>)
+                         : (wt ? &k_trace_wide<false, 1> : &k_trace_wide<false, 0>);
+        WalkerLaunch L;
+        gpugi_status st = walker_launch_config(ctx, sc, (const void*)kw, 1ull << 40, 0, L);
+        if (st) return st;
+        // a share below 100 is a stream-ordered query beside others: the wide walker then takes 70 %
+        // of it again, since its lanes refill (8 batches of 2^20 rays over four streams, 66k of them
+        // entering the scene: 541 us at the share as it is, 487 at 80-70 %, 466 at 60 %, 530 at 50 %)
+        L.grid = share_of_grid(L.grid, walkerShare < 100 ? (walkerShare * 7 + 9) / 10 : 100);
+        kw<<<L.grid, 128, 0, cs>>>(sc->dev, ox, oy, oz, dx, dy, dz, tmax, slot, t, u, v, occluded, queue, counters,
+                                   ctx->errWord);
+        GPUGI_CUDA_TRY(ctx, cudaGetLastError());
+        return GPUGI_OK;
     }
     if (ctx->traceMode >= 3) {
         auto kg = ctx->traceMode == 3

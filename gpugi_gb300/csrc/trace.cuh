@@ -587,4 +587,469 @@ GPUGI_D void group_walks_multi(uint64_t n, unsigned long long* work, uint32_t* e
     group_walks_impl<ANY_HIT, 0, G, true, 0>(DevScene{}, n, work, err, load, finish);
 }
 
+// ----------------------------------------------------------------- wide walk
+// Walks over the four-wide copy of an axis-aligned-box hierarchy (wide.cu):
+// depth first with a stack of {reference, entry distance}, children in
+// preorder, so leaves are met in exactly the order of the escape walk. The
+// results are trace_ray's bit for bit although every second level is left
+// out and four boxes are tested per fetch:
+//  * The escape walk tests a leaf's triangles iff the leaf's box and all its
+//    ancestors' boxes are hit with firstHit <= rayLength when they are met.
+//  * Boxes are nested (checked when the wide hierarchy is made) and a slab
+//    value rn(rn(plane - o) * inv) is monotone in the plane, so an
+//    ancestor's firstHit is never larger and its lastHit never smaller than
+//    the leaf's, and rayLength only shrinks. A leaf whose own test passes when
+//    it is met has ancestors that passed when they were met: the tests of
+//    the levels left out are implied. A subtree whose box fails holds no leaf
+//    that would pass.
+//  * A child that waits on the stack was tested with the rayLength of that
+//    moment; its firstHit is compared again when it is taken, which is when
+//    the escape walk would test it. So a waiting node may also be expanded
+//    early; only leaves have to be tested in order.
+//  * Monotonicity needs slab values that are not NaN. For finite rays that
+//    leaves inv = +-inf (a zero direction component) and a plane through the
+//    origin: only a box that is flat there, in a plane that also bounds an
+//    ancestor, can pass where the ancestor fails. Such a box sends the ray
+//    back to its start on the binary tree (`seq`), and non-finite rays walk
+//    the binary tree at once. (The watertight box test drops those slabs on
+//    every level, so it stays monotone.)
+//
+// What bounds it and why this split (98k-triangle room, 4.2M rays a launch,
+// ncu): L1 wavefronts 82 % busy and issue slots 70 %, DRAM idle: a lane reads
+// 112 B of node per visit, 10 visits per ray instead of 45 binary nodes. One
+// lane per ray for nodes keeps an instruction useful for ~20 lanes (8-lane
+// groups on 8-wide nodes issued 2.3x the instructions); leaves go to eight
+// lanes each, four leaves at a time, because a lane that loops over a block's
+// triangles waits for memory once per triangle (1.05 to 0.87 ms for 3M
+// any-hit rays in the 528k-triangle terrain). Quantised 96-B nodes halved
+// the L1 load but cost more issue slots than they freed (0.99 ms); prefetches
+// of waiting children cost 2-8 %.
+// Measured against the binary walkers: 3M any-hit rays in the terrain
+// 2.19 to 0.85 ms, path tracing the room at 512^2 x 16 samples 15.98 to
+// 9.5 ms, light tracing 9.16 to 5.4 ms, 1,000 rays (one per warp, the last
+// stage alone) 43 to 27 us.
+GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
+
+// Lanes of a warp step through nodes together until this many leaves wait or
+// fewer than so many lanes have a node left (leaf lanes 4 / 8 / 12: 10.09 /
+// 9.94 / 9.94 ms for the path-traced room; node lanes 4-12: the same), fetch
+// new rays when at least so many lanes are free (1 / 8 / 12 / 16: 1.04 /
+// 0.98 / 0.97 / 0.99 of the terrain's time), and hand the rays over to eight
+// lanes each when no more than two are left (0 / 2 / 4: 1.06 / 0.96 / 0.97 ms
+// for a 320 x 180 frame of one sample, whose queues end in long single walks).
+#ifndef GPUGI_WIDE_NODE_LANES
+#define GPUGI_WIDE_NODE_LANES 8
+#endif
+#ifndef GPUGI_WIDE_LEAF_LANES
+#define GPUGI_WIDE_LEAF_LANES 8
+#endif
+#ifndef GPUGI_WIDE_REFILL
+#define GPUGI_WIDE_REFILL 12
+#endif
+#ifndef GPUGI_WIDE_GROUP_AT
+#define GPUGI_WIDE_GROUP_AT 2
+#endif
+// Resident blocks per SM that the wide walkers are compiled for (64
+// registers; 7 / 8 / 9 blocks: 9.94 / 9.60 / 9.63 ms for the path-traced room).
+#ifndef GPUGI_WIDE_MIN_BLOCKS
+#define GPUGI_WIDE_MIN_BLOCKS 8
+#endif
+
+struct WideShared {
+    uint2 e[kWideShared][128];  // stack entries {reference, entry distance}, a column per ray
+    float4 ray[2][128];         // {origin, d.x}, {d.y, d.z, -, -}
+};
+
+// Persistent loop of wide walks over n work items in blocks of 128 threads:
+// the grid's warps share the first items out evenly (at most 32 each), later
+// ones come from an atomic counter *work, which starts at 0. load(i, o, d,
+// tmax) fills the ray of item i (again when a walk restarts); finish(i, slot,
+// t, u, v) takes its result (any hit: slot >= 0 when occluded). n < 2^32.
+template <bool ANY_HIT, int TRI, typename Load, typename Finish>
+GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned long long* work, uint32_t* err, Load load,
+                        Finish finish) {
+    constexpr uint32_t kNone = 0xFFFFFFFFu;  // also kWideEmpty: never a node or a leaf
+    const unsigned lane = threadIdx.x & 31u;
+    const float4* __restrict__ tris = TRI ? s.wtris : s.tris;
+    const char* __restrict__ wide = reinterpret_cast<const char*>(s.wide);
+    uint2 deep[kWideStack - kWideShared];
+    bool active = false;
+    uint32_t item = 0;
+    // -origin and 1 / direction as packed pairs
+    float2 nox = {}, noy = {}, noz = {}, ivx = {}, ivy = {}, ivz = {};
+    float len = 0.0f, u = 0.0f, v = 0.0f;
+    int32_t slot = -1;
+    uint32_t ref = kNone, sp = 0, budget = 0;
+    bool axis = false, seq = false;
+    unsigned col = threadIdx.x;  // the ray's column in shared memory
+    auto origin = [&]() { return make_float3(-nox.x, -noy.x, -noz.x); };
+    auto invdir = [&]() { return make_float3(ivx.x, ivy.x, ivz.x); };
+    auto begin = [&](uint32_t i) {
+        item = i;
+        float3 o, d;
+        load(item, o, d, len);
+        slot = -1;
+        u = v = 0.0f;
+        const float3 inv = make_float3(X::rcp(d.x), X::rcp(d.y), X::rcp(d.z));
+        sh.ray[0][col] = make_float4(o.x, o.y, o.z, d.x);
+        sh.ray[1][col] = make_float4(d.y, d.z, 0.0f, 0.0f);
+        nox = make_float2(-o.x, -o.x), noy = make_float2(-o.y, -o.y), noz = make_float2(-o.z, -o.z);
+        ivx = make_float2(inv.x, inv.x), ivy = make_float2(inv.y, inv.y), ivz = make_float2(inv.z, inv.z);
+        seq = !(finite3(o) && finite3(d));
+        axis = TRI == 0 && !finite3(inv);
+        ref = sp = 0;
+        budget = s.numNodes;
+        active = true;
+    };
+    auto pop = [&]() {  // the next pending child, or kNone
+        ref = kNone;
+        if (seq) {
+            ref = sp ? sp : kNone;
+            sp = 0;
+            return;
+        }
+        while (sp > 0) {
+            --sp;
+            uint2 e;
+            if (sp < kWideShared) e = sh.e[sp][col];
+            else e = deep[sp - kWideShared];
+            if (ANY_HIT || __uint_as_float(e.y) <= len) {
+                ref = e.x;
+                break;
+            }
+        }
+    };
+    // A node visit: every node is met once in a walk, so numNodes of them always suffice (the cap
+    // only guards against device memory corruption); checked builds test the index too.
+    auto guard = [&](uint32_t count) {
+        const bool capped = budget-- == 0, outside = kChecked && ref >= count;
+        if (capped) raise_error(err, DEVERR_TRAVERSAL_CAP);
+        if (outside) raise_error(err, DEVERR_BOUNDS);
+        if (capped || outside) {
+            ref = kNone;
+            sp = 0;
+        }
+        return capped || outside;
+    };
+    auto slots_of = [&](uint32_t leaf) {  // valid slots of a leaf word
+        const uint32_t c = (leaf >> LEAF_COUNT_SHIFT) & LEAF_COUNT_MASK;
+        if (kChecked && (uint64_t)(leaf & LEAF_BLOCK_MASK) * s.leafSize + c > s.numSlots) {
+            raise_error(err, DEVERR_BOUNDS);
+            return 0u;
+        }
+        return c;
+    };
+    auto seq_node = [&]() {  // one node of the binary tree; sp holds the escape of a hit leaf
+        const float4 a = __ldg(s.nodes + 2 * (size_t)ref), b = __ldg(s.nodes + 2 * (size_t)ref + 1);
+        float f;
+        const bool hit = intersect_box<TRI != 0>(origin(), invdir(), a, b, f) && f <= len;
+        const uint32_t child = __float_as_uint(a.w), esc = __float_as_uint(b.w);
+        if (hit && (child & LEAF_FLAG)) sp = esc;
+        ref = hit ? child : (esc ? esc : kNone);
+    };
+    // A passing box that is flat in the plane through the origin of a ray with a zero component there.
+    auto flat = [&](float3 lo, float3 hi) {
+        const float3 o = origin(), inv = invdir();
+        return (isinf(inv.x) && lo.x == o.x && hi.x == o.x) || (isinf(inv.y) && lo.y == o.y && hi.y == o.y) ||
+               (isinf(inv.z) && lo.z == o.z && hi.z == o.z);
+    };
+    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    const unsigned C = n >= 32 * (uint64_t)warps ? 32u : ((uint32_t)n + warps - 1) / warps;
+    const uint64_t first = (uint64_t)warps * C;
+    bool more = n > first;
+    {
+        const uint64_t i = ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * C + lane;
+        if (lane < C && i < n) begin((uint32_t)i);
+    }
+    // ---- a ray per lane
+    while (true) {
+        const unsigned act = __ballot_sync(0xffffffffu, active);
+        if (more && __popc(act) <= 32 - GPUGI_WIDE_REFILL) {
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(work, (unsigned long long)__popc(~act));
+            base = first + __shfl_sync(0xffffffffu, base, 0);
+            more = base + __popc(~act) < n;
+            base += (unsigned)__popc(~act & ((1u << lane) - 1u));
+            if (!active && base < n) begin((uint32_t)base);
+        } else if (!more && __popc(act) <= GPUGI_WIDE_GROUP_AT) {
+            break;
+        }
+        // nodes
+        while (true) {
+            if (active && !(ref & LEAF_FLAG)) {
+                if (guard(seq ? s.numNodes : s.numWide)) {
+                } else if (!seq) {
+                    const uint32_t at = ref * 128u;
+                    const uint32_t ax = at + (ivx.x < 0.0f ? 16u : 0u), ay = at + (ivy.x < 0.0f ? 48u : 32u),
+                                   az = at + (ivz.x < 0.0f ? 80u : 64u);
+                    auto ld = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(wide + off)); };
+                    const float4 nx = ld(ax), fx = ld(ax ^ 16u), ny = ld(ay), fy = ld(ay ^ 16u), nz = ld(az), fz = ld(az ^ 16u);
+                    const uint4 rf = __ldg(reinterpret_cast<const uint4*>(wide + (at + 96u)));
+                    // slab values of two children's planes
+                    auto slab = [](float p, float q, float2 no, float2 iv) { return __fmul2_rn(__fadd2_rn(make_float2(p, q), no), iv); };
+                    const float2 nx0 = slab(nx.x, nx.y, nox, ivx), nx1 = slab(nx.z, nx.w, nox, ivx);
+                    const float2 ny0 = slab(ny.x, ny.y, noy, ivy), ny1 = slab(ny.z, ny.w, noy, ivy);
+                    const float2 nz0 = slab(nz.x, nz.y, noz, ivz), nz1 = slab(nz.z, nz.w, noz, ivz);
+                    const float2 fx0 = slab(fx.x, fx.y, nox, ivx), fx1 = slab(fx.z, fx.w, nox, ivx);
+                    const float2 fy0 = slab(fy.x, fy.y, noy, ivy), fy1 = slab(fy.z, fy.w, noy, ivy);
+                    const float2 fz0 = slab(fz.x, fz.y, noz, ivz), fz1 = slab(fz.z, fz.w, noz, ivz);
+                    auto widen = [](float l) { return TRI ? X::mul(l, 0x1.000008p+0f) : l; };
+                    const float f0 = fmaxf(0.0f, max3f(nx0.x, ny0.x, nz0.x)), f1 = fmaxf(0.0f, max3f(nx0.y, ny0.y, nz0.y));
+                    const float f2 = fmaxf(0.0f, max3f(nx1.x, ny1.x, nz1.x)), f3 = fmaxf(0.0f, max3f(nx1.y, ny1.y, nz1.y));
+                    bool h0 = f0 <= widen(min3f(fx0.x, fy0.x, fz0.x)) && f0 <= len;
+                    bool h1 = f1 <= widen(min3f(fx0.y, fy0.y, fz0.y)) && f1 <= len;
+                    bool h2 = f2 <= widen(min3f(fx1.x, fy1.x, fz1.x)) && f2 <= len && rf.z != kWideEmpty;
+                    bool h3 = f3 <= widen(min3f(fx1.y, fy1.y, fz1.y)) && f3 <= len && rf.w != kWideEmpty;
+                    bool restart = false;
+                    if (TRI == 0 && axis) {
+                        // planes through the origin give NaN slabs: the exact test, and the binary tree
+                        // where the levels left out are not implied
+                        auto exact = [&](bool& h, float3 lo, float3 hi) {
+                            float f;
+                            h = h && intersect_box<false>(origin(), invdir(), make_float4(lo.x, lo.y, lo.z, 0.0f),
+                                                          make_float4(hi.x, hi.y, hi.z, 0.0f), f) && f <= len;
+                            restart = restart || (h && flat(lo, hi));
+                        };
+                        exact(h0, make_float3(nx.x, ny.x, nz.x), make_float3(fx.x, fy.x, fz.x));
+                        exact(h1, make_float3(nx.y, ny.y, nz.y), make_float3(fx.y, fy.y, fz.y));
+                        exact(h2, make_float3(nx.z, ny.z, nz.z), make_float3(fx.z, fy.z, fz.z));
+                        exact(h3, make_float3(nx.w, ny.w, nz.w), make_float3(fx.w, fy.w, fz.w));
+                    }
+                    // the first hit child in preorder is next, the others go on the stack, last one first
+                    const bool p1 = h1 && h0, p2 = h2 && (h0 || h1), p3 = h3 && (h0 || h1 || h2);
+                    ref = h0 ? rf.x : h1 ? rf.y : h2 ? rf.z : h3 ? rf.w : kNone;
+                    auto put = [&](bool p, uint32_t r, float f) {
+                        if (p) {
+                            if (sp < kWideShared) sh.e[sp][col] = make_uint2(r, __float_as_uint(f));
+                            else deep[sp - kWideShared] = make_uint2(r, __float_as_uint(f));
+                            ++sp;
+                        }
+                    };
+                    if (sp + 3 <= kWideShared) {  // always, but for the deepest walks
+                        uint2* e = &sh.e[sp][col];
+                        if (p3) *e = make_uint2(rf.w, __float_as_uint(f3));
+                        e += p3 ? 128 : 0;
+                        if (p2) *e = make_uint2(rf.z, __float_as_uint(f2));
+                        e += p2 ? 128 : 0;
+                        if (p1) *e = make_uint2(rf.y, __float_as_uint(f1));
+                        sp += (p3 ? 1u : 0u) + (p2 ? 1u : 0u) + (p1 ? 1u : 0u);
+                    } else {
+                        put(p3, rf.w, f3);
+                        put(p2, rf.z, f2);
+                        put(p1, rf.y, f1);
+                    }
+                    if (TRI == 0 && restart) {
+                        begin(item);
+                        seq = true;
+                    }
+                } else {
+                    seq_node();
+                }
+                if (ref == kNone) pop();
+                if (ref == kNone) {
+                    finish(item, slot, len, u, v);
+                    active = false;
+                }
+            }
+            const unsigned nodes = __ballot_sync(0xffffffffu, active && !(ref & LEAF_FLAG));
+            const unsigned leaves = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
+            if (__popc(leaves) >= GPUGI_WIDE_LEAF_LANES || __popc(nodes) < GPUGI_WIDE_NODE_LANES || !nodes) break;
+        }
+        // leaves: four at a time, eight lanes each
+        unsigned todo = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
+        __syncwarp();
+        while (todo) {
+            const unsigned my = lane >> 3, gl = lane & 7u;
+            const unsigned m1 = todo & (todo - 1), m2 = m1 & (m1 - 1), m3 = m2 & (m2 - 1);
+            const unsigned mm = my == 0 ? todo : my == 1 ? m1 : my == 2 ? m2 : m3;
+            const unsigned batch = todo & ~(m3 & (m3 - 1));
+            todo &= ~batch;
+            const unsigned src = mm ? (unsigned)(__ffs(mm) - 1) : 0u;
+            const float4 r0 = sh.ray[0][(threadIdx.x & ~31u) + src], r1 = sh.ray[1][(threadIdx.x & ~31u) + src];
+            const float3 ro = make_float3(r0.x, r0.y, r0.z), rd = make_float3(r0.w, r1.x, r1.y);
+            const uint32_t lref = __shfl_sync(0xffffffffu, ref, src);
+            WtRay w = {};
+            if (TRI) w = wt_setup(rd);
+            const bool mine = (batch >> lane) & 1u;
+            const unsigned owner = 8u * (unsigned)__popc(batch & ((1u << lane) - 1u));  // first lane of my leaf's group
+            const uint32_t k0 = (lref & LEAF_BLOCK_MASK) * s.leafSize;
+            const uint32_t cnt = mm ? slots_of(lref) : 0u;
+            for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
+                const float rl = __shfl_sync(0xffffffffu, len, src);
+                float h = 0.0f, hu = 0.0f, hv = 0.0f;
+                bool ok = false;
+                if (off < cnt) {
+                    const float4* rec = tris + 3 * (size_t)(k0 + off);
+                    const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
+                    ok = TRI ? intersect_triangle_wt_v(ro, w, a, b, c, h, hu, hv)
+                             : intersect_triangle_v(ro, rd, a, b, c, h, hu, hv);
+                    ok = ok && h < rl;
+                }
+                const unsigned any = __ballot_sync(0xffffffffu, ok);
+                if (ANY_HIT) {
+                    if (mine && (any >> (owner & 31u) & 0xffu)) slot = 0;
+                } else if (any) {
+                    const uint32_t hb = ok ? __float_as_uint(h) : 0x7fffffffu;
+                    uint32_t mn = min(hb, __shfl_xor_sync(0xffffffffu, hb, 4));
+                    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+                    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+                    const unsigned tie = __ballot_sync(0xffffffffu, ok && hb == mn);
+                    const unsigned gm = mine ? tie >> (owner & 31u) & 0xffu : 0u;
+                    const unsigned wl = gm ? owner + (unsigned)__ffs(gm) - 1 : lane;
+                    const float wh = __shfl_sync(0xffffffffu, h, wl & 31u), wu = __shfl_sync(0xffffffffu, hu, wl & 31u),
+                                wv = __shfl_sync(0xffffffffu, hv, wl & 31u);
+                    if (gm) {
+                        len = wh;
+                        u = wu;
+                        v = wv;
+                        slot = (int32_t)((ref & LEAF_BLOCK_MASK) * s.leafSize + (off - gl) + (wl & 7u));
+                    }
+                }
+            }
+            if (mine) {
+                if (ANY_HIT && slot >= 0) {
+                    ref = kNone;
+                } else {
+                    pop();
+                }
+                if (ref == kNone) {
+                    finish(item, slot, len, u, v);
+                    active = false;
+                }
+            }
+        }
+    }
+    // ---- eight lanes per ray
+    constexpr unsigned G = 8;
+    const unsigned gl = lane & (G - 1), gbase = lane & ~(G - 1), gmask = 0xffu << gbase;
+    {
+        unsigned act = __ballot_sync(0xffffffffu, active);
+        if (!act) return;
+        for (unsigned g = 0; g < lane / G; ++g) act &= act - 1;
+        const unsigned src = act ? (unsigned)(__ffs(act) - 1) : 0u;
+        auto get = [&](float x) { return __shfl_sync(0xffffffffu, x, src); };
+        auto get2 = [&](float2 x) { const float y = get(x.x); return make_float2(y, y); };
+        auto geti = [&](uint32_t x) { return __shfl_sync(0xffffffffu, x, src); };
+        nox = get2(nox), noy = get2(noy), noz = get2(noz);
+        ivx = get2(ivx), ivy = get2(ivy), ivz = get2(ivz);
+        len = get(len);
+        u = get(u);
+        v = get(v);
+        slot = (int32_t)geti((uint32_t)slot);
+        budget = geti(budget);
+        ref = geti(ref);
+        const uint32_t deepest = __reduce_max_sync(0xffffffffu, active && !seq ? sp : 0u);
+        sp = geti(sp);
+        item = geti(item);
+        axis = geti(axis) != 0;
+        seq = geti(seq) != 0;
+        col = (threadIdx.x & ~31u) + src;
+        for (uint32_t k = kWideShared; k < deepest; ++k) {
+            const uint2 e = deep[k - kWideShared];
+            deep[k - kWideShared] = make_uint2(geti(e.x), geti(e.y));
+        }
+        __syncwarp();
+        if (!act) return;
+    }
+    const float4 r0 = sh.ray[0][col], r1 = sh.ray[1][col];
+    const float3 o = make_float3(r0.x, r0.y, r0.z), d = make_float3(r0.w, r1.x, r1.y);
+    WtRay wt = {};
+    if (TRI) wt = wt_setup(d);
+    while (true) {
+        if (ref & LEAF_FLAG) {
+            const uint32_t block = ref & LEAF_BLOCK_MASK, k0 = block * s.leafSize;
+            const uint32_t cnt = slots_of(ref);
+            bool done = false;
+            for (uint32_t off = 0; off < cnt; off += G) {
+                float h = 0.0f, hu = 0.0f, hv = 0.0f;
+                bool ok = false;
+                if (off + gl < cnt) {
+                    const float4* rec = tris + 3 * (size_t)(k0 + off + gl);
+                    const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
+                    ok = TRI ? intersect_triangle_wt_v(o, wt, a, b, c, h, hu, hv)
+                             : intersect_triangle_v(o, d, a, b, c, h, hu, hv);
+                    ok = ok && h < len;
+                }
+                if (__any_sync(gmask, ok)) {
+                    if (ANY_HIT) {
+                        slot = 0;
+                        done = true;
+                        break;
+                    }
+                    const uint32_t hb = __reduce_min_sync(gmask, ok ? __float_as_uint(h) : 0x7fffffffu);
+                    const unsigned tie = __ballot_sync(gmask, ok && __float_as_uint(h) == hb);
+                    const unsigned win = (unsigned)(__ffs(tie) - 1);
+                    u = __shfl_sync(gmask, hu, win);
+                    v = __shfl_sync(gmask, hv, win);
+                    slot = (int32_t)(k0 + off + (win - gbase));
+                    len = __uint_as_float(hb);
+                }
+            }
+            ref = kNone;
+            if (done) break;
+        } else if (guard(seq ? s.numNodes : s.numWide)) {
+        } else if (!seq) {
+            // lanes 0-3: the children of `ref`; lanes 4-7: those of the next pending child if that
+            // is a node too (it is expanded early; its children are compared with rayLength when
+            // they are taken), so that a round tests two nodes
+            uint32_t mine = gl < 4 ? ref : kNone;
+            if (sp > 0 && sp <= kWideShared - 6) {
+                const uint2 e = sh.e[sp - 1][col];
+                if (!(e.x & LEAF_FLAG)) {
+                    --sp;
+                    if (gl >= 4 && (ANY_HIT || __uint_as_float(e.y) <= len)) mine = e.x;
+                }
+            }
+            bool hit = false, restart = false;
+            float f = 0.0f;
+            uint32_t r = kNone;
+            if (mine != kNone) {
+                const float* nd = reinterpret_cast<const float*>(wide + 128 * (size_t)mine) + (gl & 3u);
+                const float4 lo = make_float4(__ldg(nd), __ldg(nd + 8), __ldg(nd + 16), 0.0f);
+                const float4 hi = make_float4(__ldg(nd + 4), __ldg(nd + 12), __ldg(nd + 20), 0.0f);
+                r = __float_as_uint(__ldg(nd + 24));
+                hit = intersect_box<TRI != 0>(o, invdir(), lo, hi, f) && f <= len && r != kWideEmpty;
+                if (TRI == 0 && axis) restart = hit && flat(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z));
+            }
+            if (TRI == 0 && axis && __any_sync(gmask, restart)) {
+                begin(item);
+                seq = true;
+                continue;
+            }
+            const unsigned m = __ballot_sync(gmask, hit);
+            ref = kNone;
+            if (m) {
+                const unsigned lo = (unsigned)(__ffs(m) - 1);
+                ref = __shfl_sync(gmask, r, lo);
+                const unsigned pushes = (unsigned)__popc(m) - 1;
+                if (pushes) {
+                    if (sp + pushes <= kWideShared) {
+                        if (hit && lane != lo)
+                            sh.e[sp + __popc(m >> lane) - 1][col] = make_uint2(r, __float_as_uint(f));
+                        sp += pushes;
+                    } else {
+                        for (unsigned rest = m & (m - 1); rest;) {
+                            const unsigned top = 31u - (unsigned)__clz(rest);
+                            rest &= ~(1u << top);
+                            const uint2 e = make_uint2(__shfl_sync(gmask, r, top),
+                                                       __float_as_uint(__shfl_sync(gmask, f, top)));
+                            if (sp < kWideShared) sh.e[sp][col] = e;
+                            else deep[sp - kWideShared] = e;
+                            ++sp;
+                        }
+                    }
+                    __syncwarp(gmask);
+                }
+                continue;
+            }
+        } else {
+            seq_node();
+            if (ref != kNone) continue;
+        }
+        pop();
+        if (ref == kNone) break;
+    }
+    if (gl == 0) finish(item, slot, len, u, v);
+}
+
 }  // namespace gpugi

@@ -294,11 +294,15 @@ gpugi_status gpugi_trace_stats_device(gpugi_ctx* ctx, const gpugi_scene* scene,
  * of ceil(n / blockSize) blocks; mode 1: persistent warps that refill
  * finished lanes from a device ray counter; mode 2: a coalesced
  * root-bounds prefilter that finishes rays missing the scene and queues the
- * rest (warp-ballot compaction) for the persistent walker; modes 3
- * (default), 4 and 5: the same prefilter, then groups of 8 (mode 3), 4
- * (mode 4) or 16 (mode 5) lanes walk one ray together, testing a window of
- * consecutive preorder nodes or leaf slots per round. All modes make the same decisions per ray as TraceRay and
- * return identical results. blockSize applies to mode 0. */
+ * rest (warp-ballot compaction) for the persistent walker; mode 3
+ * (default): the same prefilter, then, on box hierarchies whose boxes nest
+ * (every one that bvhmake or gpugi_scene_build makes), a walk over a four-wide
+ * copy of the hierarchy, one lane per ray with leaves tested by eight lanes,
+ * and on other scenes groups of 8 lanes that walk one ray together, testing a
+ * window of consecutive preorder nodes or leaf slots per round; modes 4 and
+ * 5: such groups of 4 and 16 lanes on every scene. All modes make the same
+ * decisions per ray as TraceRay and return identical results. blockSize
+ * applies to mode 0. */
 gpugi_status gpugi_set_trace_config(gpugi_ctx* ctx, uint32_t mode, uint32_t blockSize);
 
 /* Host-pointer ray queries (gpugi_trace_closest / gpugi_trace_any). The

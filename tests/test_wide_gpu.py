@@ -1,0 +1,169 @@
+"""The four-wide walker (trace mode 3 on box hierarchies) against the
+one-thread-per-ray escape walk (mode 0) and the oracle: identical bits at the
+sizes and on the rays where the two could part."""
+import numpy as np
+import pytest
+
+import oracle
+from gpugi_gb300 import bvh, cuda, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = cuda.Context(0)
+    yield c
+    c.close()
+
+
+def grid_scene(n=12):
+    """Axis-aligned quads and boxes on a dyadic grid: flat leaf boxes whose planes bound their
+    ancestors, many coplanar faces."""
+    v, t = [], []
+
+    def quad(o, a, b):
+        k = len(v)
+        v.extend([o, o + a, o + a + b, o + b])
+        t.extend([[k, k + 1, k + 2, 0], [k, k + 2, k + 3, 0]])
+
+    e = np.eye(3)
+    for i in range(n):
+        for j in range(n):
+            o = np.array([i / 8, 0.0, j / 8])
+            quad(o, e[0] / 8, e[2] / 8)
+            if (i + j) % 3 == 0:
+                for a in range(3):
+                    quad(o + e[1] / 4, e[a] / 16, e[(a + 1) % 3] / 16)
+                    quad(o + e[1] / 4 + e[(a + 2) % 3] / 16, e[a] / 16, e[(a + 1) % 3] / 16)
+    return np.array(v, np.float32), np.array(t, np.uint32)
+
+
+def soup(n, seed, size):
+    """Large overlapping triangles: rays hit most boxes, so walks hold deep stacks."""
+    r = np.random.default_rng(seed)
+    c = r.uniform(-1, 1, (n, 1, 3))
+    p = (c + size * r.uniform(-1, 1, (n, 3, 3))).reshape(-1, 3).astype(np.float32)
+    t = np.concatenate([np.arange(3 * n).reshape(n, 3), np.zeros((n, 1), int)], 1).astype(np.uint32)
+    return p, t
+
+
+def make_rays(o, d, tmax):
+    a = np.concatenate([o, d, np.broadcast_to(np.asarray(tmax, np.float32).reshape(-1, 1), (len(o), 1))], 1)
+    a = np.ascontiguousarray(a.astype(np.float32).T)
+    return {k: np.ascontiguousarray(a[i]) for i, k in enumerate(cuda.RAY_KEYS)}
+
+
+def special_rays(pos, seed, n):
+    """Axis-parallel directions, origins on box planes and vertices, tiny and signed-zero components,
+    finite, zero and infinite tmax, and non-finite rays."""
+    r = np.random.default_rng(seed)
+    o = r.uniform(pos.min(0) - 0.5, pos.max(0) + 0.5, (n, 3)).astype(np.float32)
+    on = r.random((n, 3)) < 0.5
+    o = np.where(on, pos[r.integers(0, len(pos), n)], o)
+    d = r.normal(size=(n, 3)).astype(np.float32)
+    d = np.where(r.random((n, 3)) < 0.4, np.float32(0), d)
+    d = np.where(r.random((n, 3)) < 0.2, -np.abs(d) * np.float32(0), d)  # signed zeros
+    d = np.where(r.random((n, 3)) < 0.03, d * np.float32(1e-40), d)      # denormals: 1 / d overflows
+    d[np.all(d == 0, 1), 1] = -1
+    tmax = r.choice(np.array([np.inf, 3.4e38, 1.0, 0.25, 0.0, 1e-4], np.float32), n)
+    bad = r.integers(0, n, max(1, n // 50))
+    d[bad, r.integers(0, 3, len(bad))] = r.choice(np.array([np.nan, np.inf, -np.inf], np.float32), len(bad))
+    bad = r.integers(0, n, max(1, n // 50))
+    o[bad, r.integers(0, 3, len(bad))] = r.choice(np.array([np.nan, np.inf, -np.inf], np.float32), len(bad))
+    return make_rays(o, d, tmax)
+
+
+def both_modes(ctx, ds, rays):
+    got = {}
+    for mode in (3, 0):
+        ctx.set_trace_config(mode, 128)
+        got[mode] = (cuda.trace_closest(ctx, ds, rays), cuda.trace_any(ctx, ds, rays))
+    ctx.set_trace_config(3, 128)
+    return got[3], got[0]
+
+
+def same(a, b):
+    for k in ("slot", "t", "u", "v"):
+        assert np.array_equal(a[0][k].view(np.uint32), b[0][k].view(np.uint32)), k
+    assert np.array_equal(a[1], b[1])
+
+
+SCENES = {
+    "grid": lambda: grid_scene(),
+    "icosphere": lambda: (lambda s: (s["positions"], s["triangles"]))(scenes.displaced_icosphere(4096, seed=2)),
+    "soup": lambda: soup(6000, 3, 0.8),
+    "two": lambda: soup(2, 5, 1.0),
+}
+
+
+@pytest.mark.parametrize("watertight", [False, True])
+@pytest.mark.parametrize("leaf", [1, 2, 8, 32])
+@pytest.mark.parametrize("name", list(SCENES))
+def test_equals_escape_walk(ctx, name, leaf, watertight):
+    pos, tri = SCENES[name]()
+    for b in ([bvh.build_bvh(pos, tri, method="sweep", leaf_size=leaf)] if leaf != 8 else
+              [bvh.build_bvh(pos, tri, method=m, leaf_size=8) for m in ("sweep", "kdtree")]):
+        ds = ctx.upload_scene(b, pos)
+        ds.set_triangle_test(watertight)
+        for rays in (special_rays(pos, 11, 20011), scenes.aimed_rays(4099, pos, seed=6)):
+            a, z = both_modes(ctx, ds, rays)
+            same(a, z)
+        if not watertight:
+            o = oracle.trace_closest(b, pos, rays)
+            assert np.array_equal(a[0]["slot"], o["slot"])
+            assert np.array_equal(a[0]["t"].view(np.uint32), o["t"].view(np.uint32))
+            assert np.array_equal(a[1], oracle.trace_any(b, pos, rays)["occluded"])
+        ds.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 4863, 4865, 20000, 155649, 700001])
+def test_queue_lengths(ctx, n):
+    """One ray per warp, part-filled warps, one full pass of the grid, and refills."""
+    s = scenes.displaced_icosphere(16384, seed=4)
+    ds = ctx.build_scene(s["positions"], s["triangles"])
+    a, z = both_modes(ctx, ds, scenes.aimed_rays(n, s["positions"], seed=n))
+    same(a, z)
+    ds.close()
+
+
+@pytest.mark.parametrize("broken", ["not nested", "empty box", "nan box", "escape"])
+def test_trees_that_do_not_nest(ctx, broken):
+    """Hierarchies the upload accepts but the wide copy must not be made of."""
+    s = scenes.displaced_icosphere(2048, seed=7)
+    b = bvh.build_bvh(s["positions"], s["triangles"], method="sweep", leaf_size=8)
+    h = b.hierarchy.copy()
+    inner = np.nonzero((h[:, 3].view(np.uint32) & 0x80000000) == 0)[0]
+    i = inner[len(inner) // 3]
+    if broken == "not nested":
+        h[i, 0:3] = 0.6 * h[i, 0:3] + 0.4 * h[i, 4:7]
+    elif broken == "empty box":
+        h[i, [0, 4]] = h[i, [4, 0]]
+    elif broken == "nan box":
+        h[i, 5] = np.nan
+    else:  # a left child that escapes past its sibling
+        left = h[i, 3].view(np.uint32)
+        right = h[left, 7].view(np.uint32)
+        h[left, 7] = h[right, 7]
+    b.hierarchy = h
+    ds = ctx.upload_scene(b, s["positions"])
+    rays = scenes.aimed_rays(30011, s["positions"], seed=9)
+    a, z = both_modes(ctx, ds, rays)
+    same(a, z)
+    o = oracle.trace_closest(b, s["positions"], rays)
+    assert np.array_equal(a[0]["slot"], o["slot"])
+    ds.close()
+
+
+def test_chain_hierarchy(ctx):
+    """A chain deeper than the walk's stack allows (geometric spacing makes the sweep peel one leaf
+    at a time): whichever walker takes it, results are the escape walk's."""
+    r = np.random.default_rng(8)
+    x = np.cumsum(1.25 ** np.arange(160))
+    p = (r.uniform(-0.3, 0.3, (160, 3, 3)) + np.stack([x, 0 * x, 0 * x], 1)[:, None]).reshape(-1, 3).astype(np.float32)
+    t = np.concatenate([np.arange(480).reshape(160, 3), np.zeros((160, 1), int)], 1).astype(np.uint32)
+    b = bvh.build_bvh(p, t, method="sweep", leaf_size=1)
+    ds = ctx.upload_scene(b, p)
+    rays = scenes.aimed_rays(20000, p[:60], seed=3)
+    same(*both_modes(ctx, ds, rays))
+    ds.close()
