@@ -33,7 +33,8 @@ GPUGI_D uint32_t escape_word(const float4* nodes, uint32_t i) {
     return __float_as_uint(__ldg(nodes + 2 * (size_t)i + 1).w);
 }
 
-// parent[] of every child (kNoParent before), and the structure checks.
+// parent[] of every child (kNoParent before), and the structure checks (*bad
+// becomes 0 where one fails).
 __global__ void k_wide_parents(const float4* __restrict__ nodes, uint32_t n, uint32_t* parent, uint32_t* bad) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -42,13 +43,14 @@ __global__ void k_wide_parents(const float4* __restrict__ nodes, uint32_t n, uin
     const uint32_t r = c < n ? escape_word(nodes, c) : 0u;
     bool ok = c > i && c < n && r > c && r < n && escape_word(nodes, r) == escape_word(nodes, i);
     if (ok) ok = atomicExch(parent + c, i) == kNoParent && atomicExch(parent + r, i) == kNoParent;
-    if (!ok || (i == 0 && escape_word(nodes, 0) != 0u)) *bad = 1u;
+    if (!ok || (i == 0 && escape_word(nodes, 0) != 0u)) *bad = 0u;
 }
 
-// flag[i] = 1 for inner nodes at even depth below the root. Parents have
-// smaller indexes than their children, so the climb ends.
+// flag[i] = 1 for inner nodes at even depth below the root, flag[n] = 0;
+// *minNotDepth = ~(depth of the deepest inner node). Parents have smaller
+// indexes than their children, so the climb ends.
 __global__ void k_wide_mark(const float4* __restrict__ nodes, uint32_t n, const uint32_t* __restrict__ parent,
-                            uint32_t* __restrict__ flag, uint32_t* maxDepth) {
+                            uint32_t* __restrict__ flag, uint32_t* minNotDepth) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t depth = 0;
     if (i < n) {
@@ -63,15 +65,18 @@ __global__ void k_wide_mark(const float4* __restrict__ nodes, uint32_t n, const 
             if (v != 0) depth = 0;
         }
         flag[i] = mark ? 1u : 0u;
+    } else if (i == n) {
+        flag[n] = 0u;
     }
     depth = __reduce_max_sync(0xffffffffu, depth);
-    if ((threadIdx.x & 31u) == 0 && depth) atomicMax(maxDepth, depth);
+    if ((threadIdx.x & 31u) == 0 && depth) atomicMin(minNotDepth, ~depth);
 }
 
 __global__ void k_wide_fill(const float4* __restrict__ nodes, uint32_t n, const uint32_t* __restrict__ flag,
-                            const uint32_t* __restrict__ index, float4* __restrict__ wide, uint32_t* bad) {
+                            const uint32_t* __restrict__ index, uint32_t capacity, float4* __restrict__ wide,
+                            uint32_t* bad) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !flag[i]) return;
+    if (i >= n || !flag[i] || index[i] >= capacity) return;
     uint32_t kid[4], count = 0;
     bool ok = true;
     auto inside = [&](uint32_t outer, uint32_t inner) {
@@ -97,7 +102,7 @@ __global__ void k_wide_fill(const float4* __restrict__ nodes, uint32_t n, const 
         }
     }
     if (!ok) {
-        *bad = 1u;
+        *bad = 0u;
         return;
     }
     float* w = reinterpret_cast<float*>(wide + 8 * (size_t)index[i]);
@@ -109,7 +114,7 @@ __global__ void k_wide_fill(const float4* __restrict__ nodes, uint32_t n, const 
             b = __ldg(nodes + 2 * (size_t)kid[k] + 1);
             ref = __float_as_uint(a.w);
             if (!(ref & LEAF_FLAG)) {
-                if (!flag[kid[k]]) *bad = 1u;
+                if (!flag[kid[k]]) *bad = 0u;
                 ref = index[kid[k]];
             }
         }
@@ -132,8 +137,7 @@ gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc) {
     size_t scanBytes = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n + 1, st);
     // scratch in the context's staging buffer (kept between calls; every user of it finishes before it
-    // returns): parent, flag with a closing 0, index with the node count at [n] and {bad, max depth}
-    // behind it, scan storage
+    // returns): parent and {checks passed, ~depth}, flag, index (the node count at [n]), scan storage
     const size_t col = (4 * (size_t)n + 16 + 255) & ~size_t(255);
     if (gpugi_status gs = ensure_stage(ctx, 3 * col + scanBytes)) {
         cudaGetLastError();
@@ -141,36 +145,40 @@ gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc) {
     }
     char* scratch = static_cast<char*>(ctx->stageDev);
     uint32_t* parent = reinterpret_cast<uint32_t*>(scratch);
+    uint32_t* word = parent + n;
     uint32_t* flag = reinterpret_cast<uint32_t*>(scratch + col);
     uint32_t* index = reinterpret_cast<uint32_t*>(scratch + 2 * col);
-    uint32_t* word = index + n + 1;
-    const unsigned grid = (n + 255) / 256;
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(word, 0, 8, st));
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(flag + n, 0, 4, st));
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(parent, 0xFF, 4 * (size_t)n, st));
+    const unsigned grid = n / 256 + 1;  // covers [0, n]
+    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(parent, 0xFF, 4 * ((size_t)n + 2), st));
     k_wide_parents<<<grid, 256, 0, st>>>(sc->dev.nodes, n, parent, word);
     k_wide_mark<<<grid, 256, 0, st>>>(sc->dev.nodes, n, parent, flag, word + 1);
     GPUGI_CUDA_TRY(ctx, cub::DeviceScan::ExclusiveSum(scratch + 3 * col, scanBytes, flag, index, (int)n + 1, st));
-    uint32_t got[3];
-    GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got, index + n, 12, cudaMemcpyDeviceToHost, st));
-    GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    const uint32_t count = got[0];
-    // a walk's stack holds at most three entries per wide level
-    // and its node offsets are 32-bit bytes
-    if (got[1] || count == 0 || count >= (1u << 25) || 3 * (got[2] / 2 + 1) + kWideShared > kWideStack) return GPUGI_OK;
+    // At most every inner node is a wide one: small trees allocate for that (64 B a node), so that the
+    // host waits once; large ones read the count first.
+    uint32_t count = (n - 1) / 2;
+    if (n > (1u << 20)) {
+        GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(&count, index + n, 4, cudaMemcpyDeviceToHost, st));
+        GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        if (count > (n - 1) / 2) return GPUGI_OK;
+    }
+    if (count == 0) return GPUGI_OK;
     float4* wide = nullptr;
     if (cudaMalloc(&wide, 128 * (size_t)count) != cudaSuccess) {
         cudaGetLastError();
         return GPUGI_OK;
     }
     sc->allocations.push_back(wide);
-    k_wide_fill<<<grid, 256, 0, st>>>(sc->dev.nodes, n, flag, index, wide, word);
+    k_wide_fill<<<grid, 256, 0, st>>>(sc->dev.nodes, n, flag, index, count, wide, word);
     GPUGI_CUDA_TRY(ctx, cudaGetLastError());
-    GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got, word, 4, cudaMemcpyDeviceToHost, st));
+    uint32_t got[3];
+    GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got, word, 8, cudaMemcpyDeviceToHost, st));
+    GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got + 2, index + n, 4, cudaMemcpyDeviceToHost, st));
     GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if (got[0]) return GPUGI_OK;
+    // a walk's stack holds at most three entries per wide level, and its node offsets are 32-bit bytes
+    const bool fits = 3 * (~got[1] / 2 + 1) + kWideShared <= kWideStack && got[2] < (1u << 25);
+    if (got[0] == 0 || !fits || got[2] == 0 || got[2] > count) return GPUGI_OK;
     sc->wide = sc->dev.wide = wide;
-    sc->dev.numWide = count;
+    sc->dev.numWide = got[2];
     return GPUGI_OK;
 }
 
