@@ -1878,6 +1878,46 @@ __global__ void __launch_bounds__(128) k_batch_shadow(const RenderConst* __restr
         });
 }
 
+// The same queues when every job's scene has a wide hierarchy (wide_walks).
+__global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_batch_extend_wide(
+    const RenderConst* __restrict__ jobs, Counters* cnt, uint32_t* err, PathSoA A, HitSoA H, int depth) {
+    __shared__ WideShared sh;
+    const uint32_t n = cnt->path[depth];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&cnt->rays[0], (unsigned long long)n);
+    wide_walks<false, 0, true>(
+        sh, jobs[0].s, n, &cnt->extendWork[depth], err,
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> const DevScene* {
+            o = make_float3(A.ox[i], A.oy[i], A.oz[i]);
+            d = make_float3(A.dx[i], A.dy[i], A.dz[i]);
+            tmax = kRAY_MAX;
+            return &jobs[A.job[i]].s;
+        },
+        [&](uint32_t i, int32_t slot, float t, float u, float v) {
+            H.slot[i] = slot;
+            H.t[i] = t;
+            H.u[i] = u;
+            H.v[i] = v;
+        });
+}
+
+__global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_batch_shadow_wide(
+    const RenderConst* __restrict__ jobs, Counters* cnt, uint32_t* err, ShadowSoA Q, int depth) {
+    __shared__ WideShared sh;
+    const uint32_t n = cnt->shadow[depth];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&cnt->rays[1], (unsigned long long)n);
+    wide_walks<true, 0, true>(
+        sh, jobs[0].s, n, &cnt->shadowWork[depth], err,
+        [&](uint32_t i, float3& o, float3& d, float& tmax) -> const DevScene* {
+            o = make_float3(Q.ox[i], Q.oy[i], Q.oz[i]);
+            d = make_float3(Q.dx[i], Q.dy[i], Q.dz[i]);
+            tmax = Q.tmax[i];
+            return &jobs[Q.job[i]].s;
+        },
+        [&](uint32_t i, int32_t slot, float, float, float) {
+            if (slot < 0) splat(jobs[Q.job[i]], Q.pixel[i], make_float3(Q.cr[i], Q.cg[i], Q.cb[i]));
+        });
+}
+
 // One bounce of the phase-0 paths: PT eye paths, LT particles and BPT light
 // paths (the latter append to their job's light cache).
 __global__ void __launch_bounds__(128) k_batch_shade(const RenderConst* __restrict__ jobs, Counters* cnt,
@@ -2977,8 +3017,13 @@ gpugi_status gpugi_render_batch(gpugi_ctx* ctx, const gpugi_job* jobs, uint32_t 
         // launch shapes (no node staging: the walkers serve several scenes)
         WalkerLaunch LE, LS;
         const gpugi_scene* sc0 = jobs[fused[0].job].scene;
-        if ((st = walker_launch_config(ctx, sc0, (const void*)k_batch_extend, 1ull << 40, 0, LE)) ||
-            (st = walker_launch_config(ctx, sc0, (const void*)k_batch_shadow, 1ull << 40, 0, LS)))
+        // one walker serves the whole queue: the wide one where every scene has the hierarchy for it
+        bool wide = ctx->traceMode == 3;
+        for (const Fused& F : fused) wide = wide && jobs[F.job].scene->dev.wide;
+        const void* ke = wide ? (const void*)k_batch_extend_wide : (const void*)k_batch_extend;
+        const void* ks = wide ? (const void*)k_batch_shadow_wide : (const void*)k_batch_shadow;
+        if ((st = walker_launch_config(ctx, sc0, ke, 1ull << 40, 0, LE)) ||
+            (st = walker_launch_config(ctx, sc0, ks, 1ull << 40, 0, LS)))
             return st;
         int perSM0 = 0, perSM1 = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM0, (const void*)k_batch_shade, 128, 0);
@@ -2994,11 +3039,17 @@ gpugi_status gpugi_render_batch(gpugi_ctx* ctx, const gpugi_job* jobs, uint32_t 
             k_batch_generate<<<genBlocks, 256, 0, stream>>>(rb->dJobs, rb->dOffsets + ph * (nj + 1), nj, rb->cnt, A,
                                                             rb->Q, ph);
             for (int depth = 0; depth < (int)maxDepth; ++depth) {
-                k_batch_extend<<<LE.grid, 128, 0, stream>>>(rb->dJobs, rb->cnt, ctx->errWord, A, rb->H, depth,
-                                                            groupE);
+                if (wide)
+                    k_batch_extend_wide<<<LE.grid, 128, 0, stream>>>(rb->dJobs, rb->cnt, ctx->errWord, A, rb->H, depth);
+                else
+                    k_batch_extend<<<LE.grid, 128, 0, stream>>>(rb->dJobs, rb->cnt, ctx->errWord, A, rb->H, depth,
+                                                                groupE);
                 if (ph == 0) k_batch_shade<<<gridShade0, 128, 0, stream>>>(rb->dJobs, rb->cnt, A, B, rb->H, rb->Q, depth);
                 else k_batch_bpt_shade<<<gridShade1, 128, 0, stream>>>(rb->dJobs, rb->cnt, A, B, rb->H, rb->Q, depth);
-                k_batch_shadow<<<LS.grid, 128, 0, stream>>>(rb->dJobs, rb->cnt, ctx->errWord, rb->Q, depth, groupS);
+                if (wide)
+                    k_batch_shadow_wide<<<LS.grid, 128, 0, stream>>>(rb->dJobs, rb->cnt, ctx->errWord, rb->Q, depth);
+                else
+                    k_batch_shadow<<<LS.grid, 128, 0, stream>>>(rb->dJobs, rb->cnt, ctx->errWord, rb->Q, depth, groupS);
                 std::swap(A, B);
             }
         };
@@ -3009,7 +3060,7 @@ gpugi_status gpugi_render_batch(gpugi_ctx* ctx, const gpugi_job* jobs, uint32_t 
         if (ctx->batchGraph) {
             const std::vector<uintptr_t> key = {(uintptr_t)rb->block, (uintptr_t)rb->dJobs, nj, depth0, depth1,
                                                 LE.grid, LS.grid, gridShade0, gridShade1, (uintptr_t)ctx->errWord,
-                                                groupE, groupS};
+                                                groupE, groupS, wide};
             if (!rb->batchExec || key != rb->batchKey) {
                 if (rb->batchExec) cudaGraphExecDestroy(rb->batchExec);
                 rb->batchExec = nullptr;

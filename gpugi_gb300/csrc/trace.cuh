@@ -665,13 +665,21 @@ struct WideShared {
 // ones come from an atomic counter *work, which starts at 0. load(i, o, d,
 // tmax) fills the ray of item i (again when a walk restarts); finish(i, slot,
 // t, u, v) takes its result (any hit: slot >= 0 when occluded). n < 2^32.
-template <bool ANY_HIT, int TRI, typename Load, typename Finish>
-GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned long long* work, uint32_t* err, Load load,
+// MULTI: the items belong to several scenes, load returns the item's (a scene
+// with a wide hierarchy); otherwise every ray walks `scene`.
+template <bool ANY_HIT, int TRI, bool MULTI = false, typename Load, typename Finish>
+GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsigned long long* work, uint32_t* err, Load load,
                         Finish finish) {
     constexpr uint32_t kNone = 0xFFFFFFFFu;  // also kWideEmpty: never a node or a leaf
     const unsigned lane = threadIdx.x & 31u;
-    const float4* __restrict__ tris = TRI ? s.wtris : s.tris;
-    const char* __restrict__ wide = reinterpret_cast<const char*>(s.wide);
+    const DevScene* own = &scene;  // MULTI: the scene of the lane's ray
+    const char* wide = reinterpret_cast<const char*>(scene.wide);
+    auto tris_of = [](const DevScene& s) { return TRI ? s.wtris : s.tris; };
+    auto shfl_scene = [&](unsigned mask, unsigned src) {
+        const uint64_t p = reinterpret_cast<uint64_t>(own);
+        return reinterpret_cast<const DevScene*>((uint64_t)__shfl_sync(mask, (uint32_t)(p >> 32), src) << 32 |
+                                                 __shfl_sync(mask, (uint32_t)p, src));
+    };
     uint2 deep[kWideStack - kWideShared];
     bool active = false;
     uint32_t item = 0;
@@ -687,7 +695,12 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
     auto begin = [&](uint32_t i) {
         item = i;
         float3 o, d;
-        load(item, o, d, len);
+        if constexpr (MULTI) {
+            own = load(item, o, d, len);
+            wide = reinterpret_cast<const char*>(own->wide);
+        } else {
+            load(item, o, d, len);
+        }
         slot = -1;
         u = v = 0.0f;
         const float3 inv = make_float3(X::rcp(d.x), X::rcp(d.y), X::rcp(d.z));
@@ -698,7 +711,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
         seq = !(finite3(o) && finite3(d));
         axis = TRI == 0 && !finite3(inv);
         ref = sp = 0;
-        budget = s.numNodes;
+        budget = own->numNodes;
         active = true;
     };
     auto pop = [&]() {  // the next pending child, or kNone
@@ -731,7 +744,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
         }
         return capped || outside;
     };
-    auto slots_of = [&](uint32_t leaf) {  // valid slots of a leaf word
+    auto slots_of = [&](const DevScene& s, uint32_t leaf) {  // valid slots of a leaf word
         const uint32_t c = (leaf >> LEAF_COUNT_SHIFT) & LEAF_COUNT_MASK;
         if (kChecked && (uint64_t)(leaf & LEAF_BLOCK_MASK) * s.leafSize + c > s.numSlots) {
             raise_error(err, DEVERR_BOUNDS);
@@ -740,7 +753,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
         return c;
     };
     auto seq_node = [&]() {  // one node of the binary tree; sp holds the escape of a hit leaf
-        const float4 a = __ldg(s.nodes + 2 * (size_t)ref), b = __ldg(s.nodes + 2 * (size_t)ref + 1);
+        const float4 a = __ldg(own->nodes + 2 * (size_t)ref), b = __ldg(own->nodes + 2 * (size_t)ref + 1);
         float f;
         const bool hit = intersect_box<TRI != 0>(origin(), invdir(), a, b, f) && f <= len;
         const uint32_t child = __float_as_uint(a.w), esc = __float_as_uint(b.w);
@@ -777,7 +790,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
         // nodes
         while (true) {
             if (active && !(ref & LEAF_FLAG)) {
-                if (guard(seq ? s.numNodes : s.numWide)) {
+                if (guard(seq ? own->numNodes : own->numWide)) {
                 } else if (!seq) {
                     const uint32_t at = ref * 128u;
                     const uint32_t ax = at + (ivx.x < 0.0f ? 16u : 0u), ay = at + (ivy.x < 0.0f ? 48u : 32u),
@@ -868,18 +881,19 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
             const float4 r0 = sh.ray[0][(threadIdx.x & ~31u) + src], r1 = sh.ray[1][(threadIdx.x & ~31u) + src];
             const float3 ro = make_float3(r0.x, r0.y, r0.z), rd = make_float3(r0.w, r1.x, r1.y);
             const uint32_t lref = __shfl_sync(0xffffffffu, ref, src);
+            const DevScene* ls = MULTI ? shfl_scene(0xffffffffu, src) : own;
             WtRay w = {};
             if (TRI) w = wt_setup(rd);
             const bool mine = (batch >> lane) & 1u;
             const unsigned owner = 8u * (unsigned)__popc(batch & ((1u << lane) - 1u));  // first lane of my leaf's group
-            const uint32_t k0 = (lref & LEAF_BLOCK_MASK) * s.leafSize;
-            const uint32_t cnt = mm ? slots_of(lref) : 0u;
+            const uint32_t k0 = mm ? (lref & LEAF_BLOCK_MASK) * ls->leafSize : 0u;
+            const uint32_t cnt = mm ? slots_of(*ls, lref) : 0u;
             for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
                 const float rl = __shfl_sync(0xffffffffu, len, src);
                 float h = 0.0f, hu = 0.0f, hv = 0.0f;
                 bool ok = false;
                 if (off < cnt) {
-                    const float4* rec = tris + 3 * (size_t)(k0 + off);
+                    const float4* rec = tris_of(*ls) + 3 * (size_t)(k0 + off);
                     const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
                     ok = TRI ? intersect_triangle_wt_v(ro, w, a, b, c, h, hu, hv)
                              : intersect_triangle_v(ro, rd, a, b, c, h, hu, hv);
@@ -902,7 +916,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
                         len = wh;
                         u = wu;
                         v = wv;
-                        slot = (int32_t)((ref & LEAF_BLOCK_MASK) * s.leafSize + (off - gl) + (wl & 7u));
+                        slot = (int32_t)((ref & LEAF_BLOCK_MASK) * own->leafSize + (off - gl) + (wl & 7u));
                     }
                 }
             }
@@ -949,6 +963,10 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
             deep[k - kWideShared] = make_uint2(geti(e.x), geti(e.y));
         }
         __syncwarp();
+        if (MULTI) {
+            own = shfl_scene(0xffffffffu, src);
+            wide = reinterpret_cast<const char*>(own->wide);
+        }
         if (!act) return;
     }
     const float4 r0 = sh.ray[0][col], r1 = sh.ray[1][col];
@@ -957,14 +975,14 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
     if (TRI) wt = wt_setup(d);
     while (true) {
         if (ref & LEAF_FLAG) {
-            const uint32_t block = ref & LEAF_BLOCK_MASK, k0 = block * s.leafSize;
-            const uint32_t cnt = slots_of(ref);
+            const uint32_t block = ref & LEAF_BLOCK_MASK, k0 = block * own->leafSize;
+            const uint32_t cnt = slots_of(*own, ref);
             bool done = false;
             for (uint32_t off = 0; off < cnt; off += G) {
                 float h = 0.0f, hu = 0.0f, hv = 0.0f;
                 bool ok = false;
                 if (off + gl < cnt) {
-                    const float4* rec = tris + 3 * (size_t)(k0 + off + gl);
+                    const float4* rec = tris_of(*own) + 3 * (size_t)(k0 + off + gl);
                     const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
                     ok = TRI ? intersect_triangle_wt_v(o, wt, a, b, c, h, hu, hv)
                              : intersect_triangle_v(o, d, a, b, c, h, hu, hv);
@@ -987,7 +1005,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& s, uint64_t n, unsigned 
             }
             ref = kNone;
             if (done) break;
-        } else if (guard(seq ? s.numNodes : s.numWide)) {
+        } else if (guard(seq ? own->numNodes : own->numWide)) {
         } else if (!seq) {
             // lanes 0-3: the children of `ref`; lanes 4-7: those of the next pending child if that
             // is a node too (it is expanded early; its children are compared with rayLength when

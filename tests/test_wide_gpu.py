@@ -167,3 +167,36 @@ def test_chain_hierarchy(ctx):
     rays = scenes.aimed_rays(20000, p[:60], seed=3)
     same(*both_modes(ctx, ds, rays))
     ds.close()
+
+
+@pytest.mark.parametrize("size,samples", [(7, 1), (64, 1), (200, 5)])
+def test_passes_and_batches(ctx, size, samples):
+    """PT and LT images, singly and batched over two scenes, against the same calls on the binary
+    walkers (trace mode 2): the same paths, so images differ only by the order of at most a few
+    hundred float additions per pixel (2^-24 each, on sums of non-negative terms)."""
+    from gpugi_gb300 import render
+    sets = []
+    for level, grid in ((3, 6), (2, 4)):
+        s = scenes.cornell_room(seed=1, sphere_level=level, wall_grid=grid)
+        b = bvh.build_bvh(s["positions"], s["triangles"], method="sweep")
+        sets.append(ctx.upload_scene(b, s["positions"], cuda.vertex_info(s["normals"], s["texcoords"]), s["materials"]))
+    cam = render.camera_lookat(*scenes.CORNELL_CAMERA, size, size)
+    images = {}
+    for mode in (2, 3):
+        ctx.set_trace_config(mode, 128)
+        out = []
+        for pass_ in ("PT", "LT"):
+            img = render.Image(ctx, size, size)
+            render.render(ctx, sets[0], cam, img, pass_, max_path_length=6, samples=samples, rng_state=[5])
+            out.append(img.read())
+        jobs = [dict(scene=sets[k % 2], camera=cam, image=render.Image(ctx, size, size), pass_=("PT", "LT", "PT")[k],
+                     samples=samples, max_path_length=6, rng_state=[7 + k]) for k in range(3)]
+        render.render_batch(ctx, jobs)
+        out += [j["image"].read() for j in jobs]
+        images[mode] = out
+    ctx.set_trace_config(3, 128)
+    for a, z in zip(images[3], images[2]):
+        assert z[..., :3].any()
+        assert np.abs(a - z).max() <= 512 * 2.0 ** -24 * max(1.0, float(np.abs(z).max()))
+    for s in sets:
+        s.close()
