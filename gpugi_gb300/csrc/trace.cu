@@ -317,8 +317,7 @@ __global__ void __launch_bounds__(128) k_trace_queue(
     }
 }
 
-// Group walker (modes 4 and 5, and mode 3 on scenes without a wide hierarchy),
-// second launch after the root prefilter: G
+// Group walker (modes 4 and 5), second launch after the root prefilter: G
 // lanes walk each queued ray together (group_step), which shortens the
 // dependent fetch chain of the longest walks.
 template <bool ANY_HIT, int BOUNDS, int G, int TRI>
@@ -378,6 +377,42 @@ __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide(
                 v[ray] = hitV;
             }
         });
+}
+
+// Second launch of mode 3 on scenes without a wide hierarchy: 8-lane groups
+// for short queues, one lane per ray for long ones.
+template <bool ANY_HIT, int BOUNDS, int TRI>
+__global__ void __launch_bounds__(128, 8) k_trace_binary(
+    DevScene s, const float* __restrict__ ox, const float* __restrict__ oy, const float* __restrict__ oz,
+    const float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ dz,
+    const float* __restrict__ tmax, int32_t* __restrict__ slot, float* __restrict__ t, float* __restrict__ u,
+    float* __restrict__ v, uint8_t* __restrict__ occluded, const uint32_t* __restrict__ queue,
+    unsigned long long* counters, uint32_t* err) {
+    __shared__ LaneShared sh;
+    const uint64_t n = counters[1];
+    auto load = [&](uint64_t i, float3& o, float3& d, float& len) {
+        const uint32_t ray = __ldg(queue + i);
+        o = make_float3(__ldg(ox + ray), __ldg(oy + ray), __ldg(oz + ray));
+        d = make_float3(__ldg(dx + ray), __ldg(dy + ray), __ldg(dz + ray));
+        len = __ldg(tmax + ray);
+    };
+    auto finish = [&](uint64_t i, int32_t hitSlot, float hitT, float hitU, float hitV) {
+        const uint32_t ray = __ldg(queue + i);
+        if (ANY_HIT) {
+            occluded[ray] = hitSlot >= 0 ? 1 : 0;
+        } else {
+            slot[ray] = hitSlot;
+            t[ray] = hitT;
+            u[ray] = hitU;
+            v[ray] = hitV;
+        }
+    };
+    if (n < (uint64_t)gridDim.x * GPUGI_LANE_FROM)
+        group_walks<ANY_HIT, BOUNDS, 8, TRI>(s, n, counters + 2, err, load, [&](uint64_t i, const GroupWalk& g) {
+            finish(i, g.slot, g.len, g.u, g.v);
+        });
+    else
+        lane_walks<ANY_HIT, BOUNDS, TRI>(sh, s, n, counters + 2, err, load, finish);
 }
 
 // walkerShare percent of a persistent walker grid (at least one block).
@@ -458,7 +493,7 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
     if (ctx->traceMode >= 3) {
         auto kg = ctx->traceMode == 3
                       ? pick_variant(anyHit, ell, wt, [](auto A, auto B, auto T) {
-                            return &k_trace_group<decltype(A)::value, decltype(B)::value, 8, decltype(T)::value>;
+                            return &k_trace_binary<decltype(A)::value, decltype(B)::value, decltype(T)::value>;
                         })
                   : ctx->traceMode == 4
                       ? pick_variant(anyHit, ell, wt, [](auto A, auto B, auto T) {

@@ -660,6 +660,80 @@ struct WideShared {
     float4 ray[2][128];         // {origin, d.x}, {d.y, d.z, -, -}
 };
 
+// Valid slots of a leaf word (checked builds: none where they pass the end).
+GPUGI_D uint32_t leaf_slots(const DevScene& s, uint32_t leaf, uint32_t* err) {
+    const uint32_t c = (leaf >> LEAF_COUNT_SHIFT) & LEAF_COUNT_MASK;
+    if (kChecked && (uint64_t)(leaf & LEAF_BLOCK_MASK) * s.leafSize + c > s.numSlots) {
+        raise_error(err, DEVERR_BOUNDS);
+        return 0u;
+    }
+    return c;
+}
+
+// The leaves of the lanes in `todo` (each holds a leaf word in ref), four at a
+// time by eight lanes each; the rays come from shared memory (ray[.][thread]
+// = {origin, d.x}, {d.y, d.z, -, -}). A leaf's result is the sequential rule's:
+// the first slot reaching the minimum hit distance below the owner's len (any
+// hit: slot becomes 0 when a triangle is accepted). scene_of(lane) is the
+// scene of a lane's ray, own the caller's; after() runs in the owner.
+template <bool ANY_HIT, int TRI, typename SceneOf, typename After>
+GPUGI_D void leaf_rounds(unsigned todo, const float4 (*ray)[128], const uint32_t& ref, SceneOf scene_of,
+                         const DevScene* const& own, uint32_t* err, float& len, float& u, float& v, int32_t& slot,
+                         After after) {
+    const unsigned lane = threadIdx.x & 31u;
+    while (todo) {
+        const unsigned my = lane >> 3, gl = lane & 7u;
+        const unsigned m1 = todo & (todo - 1), m2 = m1 & (m1 - 1), m3 = m2 & (m2 - 1);
+        const unsigned mm = my == 0 ? todo : my == 1 ? m1 : my == 2 ? m2 : m3;
+        const unsigned batch = todo & ~(m3 & (m3 - 1));
+        todo &= ~batch;
+        const unsigned src = mm ? (unsigned)(__ffs(mm) - 1) : 0u;
+        const float4 r0 = ray[0][(threadIdx.x & ~31u) + src], r1 = ray[1][(threadIdx.x & ~31u) + src];
+        const float3 ro = make_float3(r0.x, r0.y, r0.z), rd = make_float3(r0.w, r1.x, r1.y);
+        const uint32_t lref = __shfl_sync(0xffffffffu, ref, src);
+        const DevScene* ls = scene_of(src);
+        WtRay w = {};
+        if (TRI) w = wt_setup(rd);
+        const bool mine = (batch >> lane) & 1u;
+        const unsigned owner = 8u * (unsigned)__popc(batch & ((1u << lane) - 1u));  // first lane of my leaf's group
+        const uint32_t k0 = mm ? (lref & LEAF_BLOCK_MASK) * ls->leafSize : 0u;
+        const uint32_t cnt = mm ? leaf_slots(*ls, lref, err) : 0u;
+        for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
+            const float rl = __shfl_sync(0xffffffffu, len, src);
+            float h = 0.0f, hu = 0.0f, hv = 0.0f;
+            bool ok = false;
+            if (off < cnt) {
+                const float4* rec = (TRI ? ls->wtris : ls->tris) + 3 * (size_t)(k0 + off);
+                const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
+                ok = TRI ? intersect_triangle_wt_v(ro, w, a, b, c, h, hu, hv)
+                         : intersect_triangle_v(ro, rd, a, b, c, h, hu, hv);
+                ok = ok && h < rl;
+            }
+            const unsigned any = __ballot_sync(0xffffffffu, ok);
+            if (ANY_HIT) {
+                if (mine && (any >> (owner & 31u) & 0xffu)) slot = 0;
+            } else if (any) {
+                const uint32_t hb = ok ? __float_as_uint(h) : 0x7fffffffu;
+                uint32_t mn = min(hb, __shfl_xor_sync(0xffffffffu, hb, 4));
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+                const unsigned tie = __ballot_sync(0xffffffffu, ok && hb == mn);
+                const unsigned gm = mine ? tie >> (owner & 31u) & 0xffu : 0u;
+                const unsigned wl = gm ? owner + (unsigned)__ffs(gm) - 1 : lane;
+                const float wh = __shfl_sync(0xffffffffu, h, wl & 31u), wu = __shfl_sync(0xffffffffu, hu, wl & 31u),
+                            wv = __shfl_sync(0xffffffffu, hv, wl & 31u);
+                if (gm) {
+                    len = wh;
+                    u = wu;
+                    v = wv;
+                    slot = (int32_t)((ref & LEAF_BLOCK_MASK) * own->leafSize + (off - gl) + (wl & 7u));
+                }
+            }
+        }
+        if (mine) after();
+    }
+}
+
 // Persistent loop of wide walks over n work items in blocks of 128 threads:
 // the grid's warps share the first items out evenly (at most 32 each), later
 // ones come from an atomic counter *work, which starts at 0. load(i, o, d,
@@ -743,14 +817,6 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
             sp = 0;
         }
         return capped || outside;
-    };
-    auto slots_of = [&](const DevScene& s, uint32_t leaf) {  // valid slots of a leaf word
-        const uint32_t c = (leaf >> LEAF_COUNT_SHIFT) & LEAF_COUNT_MASK;
-        if (kChecked && (uint64_t)(leaf & LEAF_BLOCK_MASK) * s.leafSize + c > s.numSlots) {
-            raise_error(err, DEVERR_BOUNDS);
-            return 0u;
-        }
-        return c;
     };
     auto seq_node = [&]() {  // one node of the binary tree; sp holds the escape of a hit leaf
         const float4 a = __ldg(own->nodes + 2 * (size_t)ref), b = __ldg(own->nodes + 2 * (size_t)ref + 1);
@@ -871,56 +937,9 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
         // leaves: four at a time, eight lanes each
         unsigned todo = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
         __syncwarp();
-        while (todo) {
-            const unsigned my = lane >> 3, gl = lane & 7u;
-            const unsigned m1 = todo & (todo - 1), m2 = m1 & (m1 - 1), m3 = m2 & (m2 - 1);
-            const unsigned mm = my == 0 ? todo : my == 1 ? m1 : my == 2 ? m2 : m3;
-            const unsigned batch = todo & ~(m3 & (m3 - 1));
-            todo &= ~batch;
-            const unsigned src = mm ? (unsigned)(__ffs(mm) - 1) : 0u;
-            const float4 r0 = sh.ray[0][(threadIdx.x & ~31u) + src], r1 = sh.ray[1][(threadIdx.x & ~31u) + src];
-            const float3 ro = make_float3(r0.x, r0.y, r0.z), rd = make_float3(r0.w, r1.x, r1.y);
-            const uint32_t lref = __shfl_sync(0xffffffffu, ref, src);
-            const DevScene* ls = MULTI ? shfl_scene(0xffffffffu, src) : own;
-            WtRay w = {};
-            if (TRI) w = wt_setup(rd);
-            const bool mine = (batch >> lane) & 1u;
-            const unsigned owner = 8u * (unsigned)__popc(batch & ((1u << lane) - 1u));  // first lane of my leaf's group
-            const uint32_t k0 = mm ? (lref & LEAF_BLOCK_MASK) * ls->leafSize : 0u;
-            const uint32_t cnt = mm ? slots_of(*ls, lref) : 0u;
-            for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
-                const float rl = __shfl_sync(0xffffffffu, len, src);
-                float h = 0.0f, hu = 0.0f, hv = 0.0f;
-                bool ok = false;
-                if (off < cnt) {
-                    const float4* rec = tris_of(*ls) + 3 * (size_t)(k0 + off);
-                    const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
-                    ok = TRI ? intersect_triangle_wt_v(ro, w, a, b, c, h, hu, hv)
-                             : intersect_triangle_v(ro, rd, a, b, c, h, hu, hv);
-                    ok = ok && h < rl;
-                }
-                const unsigned any = __ballot_sync(0xffffffffu, ok);
-                if (ANY_HIT) {
-                    if (mine && (any >> (owner & 31u) & 0xffu)) slot = 0;
-                } else if (any) {
-                    const uint32_t hb = ok ? __float_as_uint(h) : 0x7fffffffu;
-                    uint32_t mn = min(hb, __shfl_xor_sync(0xffffffffu, hb, 4));
-                    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
-                    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
-                    const unsigned tie = __ballot_sync(0xffffffffu, ok && hb == mn);
-                    const unsigned gm = mine ? tie >> (owner & 31u) & 0xffu : 0u;
-                    const unsigned wl = gm ? owner + (unsigned)__ffs(gm) - 1 : lane;
-                    const float wh = __shfl_sync(0xffffffffu, h, wl & 31u), wu = __shfl_sync(0xffffffffu, hu, wl & 31u),
-                                wv = __shfl_sync(0xffffffffu, hv, wl & 31u);
-                    if (gm) {
-                        len = wh;
-                        u = wu;
-                        v = wv;
-                        slot = (int32_t)((ref & LEAF_BLOCK_MASK) * own->leafSize + (off - gl) + (wl & 7u));
-                    }
-                }
-            }
-            if (mine) {
+        leaf_rounds<ANY_HIT, TRI>(
+            todo, sh.ray, ref, [&](unsigned src) { return MULTI ? shfl_scene(0xffffffffu, src) : own; }, own, err, len, u,
+            v, slot, [&]() {
                 if (ANY_HIT && slot >= 0) {
                     ref = kNone;
                 } else {
@@ -930,8 +949,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     finish(item, slot, len, u, v);
                     active = false;
                 }
-            }
-        }
+            });
     }
     // ---- eight lanes per ray
     constexpr unsigned G = 8;
@@ -976,7 +994,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
     while (true) {
         if (ref & LEAF_FLAG) {
             const uint32_t block = ref & LEAF_BLOCK_MASK, k0 = block * own->leafSize;
-            const uint32_t cnt = slots_of(*own, ref);
+            const uint32_t cnt = leaf_slots(*own, ref, err);
             bool done = false;
             for (uint32_t off = 0; off < cnt; off += G) {
                 float h = 0.0f, hu = 0.0f, hv = 0.0f;
@@ -1068,6 +1086,154 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
         if (ref == kNone) break;
     }
     if (gl == 0) finish(item, slot, len, u, v);
+}
+
+// ----------------------------------------------------------------- lane walk
+// The escape walk of the binary tree, one lane per ray, for trees that have no
+// wide hierarchy (ellipsoids and oriented boxes: their bounds do not nest, so
+// every ancestor has to be tested) and queues that are long enough: lanes
+// step through nodes together, leaves are tested by eight lanes each as in
+// wide_walks, and the last rays of a warp continue as 8-lane groups
+// (group_step), whose windows shorten the long single walks that a queue
+// ends with. Same items, load and finish as wide_walks.
+//
+// Bound by issue slots (an ellipsoid test is ~70 instructions with a
+// reciprocal and a square root): 8-lane groups issued ~2,700 instructions per
+// ray for windows of which a third is visited. Measured on fitted ellipsoids,
+// 100k instanced triangles, rays from inside (us, 8-lane groups / this):
+// 20,000 rays 143 / 158, 40,000 181 / 199, 60,000 209 / 216, 100,000 281 / 240,
+// 500,000 935 / 458, 2,000,000 3,451 / 1,349. So queues of fewer rays than
+// 56 per block of the full grid (68,000 on 152 SMs) stay with the groups.
+// Nodes per loop 1 / 2 / 4 / 8: 496 / 489 / 458 / 473 us at 500,000; waiting
+// leaves 2 / 4 / 8: 462 / 458 / 476; handed over at 2 / 3 / 4 rays: 509 / 471
+// / 458.
+#ifndef GPUGI_LANE_FROM
+#define GPUGI_LANE_FROM 56u
+#endif
+constexpr int kLaneSteps = 4, kLaneLeaves = 4, kLaneNodes = 8, kLaneRefill = 8, kLaneGroupAt = 4;
+struct LaneShared {
+    float4 ray[2][128];
+};
+
+template <bool ANY_HIT, int BOUNDS, int TRI, typename Load, typename Finish>
+GPUGI_D void lane_walks(LaneShared& sh, const DevScene& s, uint64_t n, unsigned long long* work, uint32_t* err,
+                        Load load, Finish finish) {
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    const unsigned lane = threadIdx.x & 31u;
+    const DevScene* const own = &s;
+    bool active = false;
+    uint32_t item = 0;
+    float3 o = {}, d = {}, inv = {};
+    float len = 0.0f, u = 0.0f, v = 0.0f;
+    int32_t slot = -1;
+    uint32_t ref = kNone, resume = kNone, budget = 0;  // ref: node or leaf word to take next; resume: after a leaf
+    auto begin = [&](uint32_t i) {
+        item = i;
+        load(item, o, d, len);
+        slot = -1;
+        u = v = 0.0f;
+        inv = make_float3(X::rcp(d.x), X::rcp(d.y), X::rcp(d.z));
+        sh.ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, d.x);
+        sh.ray[1][threadIdx.x] = make_float4(d.y, d.z, 0.0f, 0.0f);
+        ref = 0;
+        budget = s.numNodes;
+        active = true;
+    };
+    auto step = [&]() {  // one node
+        const bool capped = budget-- == 0, outside = kChecked && ref >= s.numNodes;
+        if (capped || outside) {
+            raise_error(err, capped ? DEVERR_TRAVERSAL_CAP : DEVERR_BOUNDS);
+            ref = kNone;
+            return;
+        }
+        const float4* nd = s.nodes + node_stride<BOUNDS>() * (size_t)ref;
+        const float4 a = __ldg(nd), b = __ldg(nd + 1);
+        const float4 c = BOUNDS == 2 ? __ldg(nd + 2) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float f;
+        const bool hit = bounds_test<BOUNDS, TRI != 0>(o, d, inv, a, b, c, f) && f <= len;
+        const uint32_t child = __float_as_uint(a.w), esc = __float_as_uint(b.w), next = esc ? esc : kNone;
+        if (hit && (child & LEAF_FLAG)) resume = next;
+        ref = hit ? child : next;
+    };
+    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    const unsigned C = n >= 32 * (uint64_t)warps ? 32u : ((uint32_t)n + warps - 1) / warps;
+    const uint64_t first = (uint64_t)warps * C;
+    bool more = n > first;
+    {
+        const uint64_t i = ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * C + lane;
+        if (lane < C && i < n) begin((uint32_t)i);
+    }
+    while (true) {
+        const unsigned act = __ballot_sync(0xffffffffu, active);
+        if (more && __popc(act) <= 32 - kLaneRefill) {
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(work, (unsigned long long)__popc(~act));
+            base = first + __shfl_sync(0xffffffffu, base, 0);
+            more = base + __popc(~act) < n;
+            base += (unsigned)__popc(~act & ((1u << lane) - 1u));
+            if (!active && base < n) begin((uint32_t)base);
+        } else if (!more && __popc(act) <= kLaneGroupAt) {
+            break;
+        }
+        // nodes
+        while (true) {
+            if (active && !(ref & LEAF_FLAG)) {
+#pragma unroll 1
+                for (int k = 0; k < kLaneSteps && !(ref & LEAF_FLAG); ++k) step();
+                if (ref == kNone) {
+                    finish(item, slot, len, u, v);
+                    active = false;
+                }
+            }
+            const unsigned nodes = __ballot_sync(0xffffffffu, active && !(ref & LEAF_FLAG));
+            const unsigned leaves = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
+            if (__popc(leaves) >= kLaneLeaves || __popc(nodes) < kLaneNodes || !nodes) break;
+        }
+        const unsigned todo = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
+        __syncwarp();
+        leaf_rounds<ANY_HIT, TRI>(todo, sh.ray, ref, [&](unsigned) { return own; }, own, err, len, u, v, slot, [&]() {
+            ref = ANY_HIT && slot >= 0 ? kNone : resume;
+            if (ref == kNone) {
+                finish(item, slot, len, u, v);
+                active = false;
+            }
+        });
+    }
+    // the last rays: eight lanes each
+    constexpr unsigned G = 8;
+    const unsigned gl = lane & (G - 1), gbase = lane & ~(G - 1), gmask = 0xffu << gbase;
+    unsigned act = __ballot_sync(0xffffffffu, active);
+    for (unsigned g = 0; g < lane / G; ++g) act &= act - 1;
+    const unsigned src = act ? (unsigned)(__ffs(act) - 1) : 0u;
+    auto get = [&](float x) { return __shfl_sync(0xffffffffu, x, src); };
+    GroupWalk g;
+    g.o = make_float3(get(o.x), get(o.y), get(o.z));
+    g.d = make_float3(get(d.x), get(d.y), get(d.z));
+    g.inv = make_float3(get(inv.x), get(inv.y), get(inv.z));
+    g.wt = wt_setup(g.d);  // dead code unless a watertight walker reads it
+    g.len = get(len);
+    g.u = get(u);
+    g.v = get(v);
+    g.slot = __shfl_sync(0xffffffffu, slot, src);
+    g.budget = __shfl_sync(0xffffffffu, budget, src);
+    item = __shfl_sync(0xffffffffu, item, src);
+    ref = __shfl_sync(0xffffffffu, ref, src);
+    resume = __shfl_sync(0xffffffffu, resume, src);
+    if (!act) return;
+    g.node = ref;
+    g.cur = g.end = 0;
+    g.resume = resume;
+    bool done = false;
+    if (ref & LEAF_FLAG) {
+        g.cur = (ref & LEAF_BLOCK_MASK) * s.leafSize;
+        g.end = g.cur + leaf_slots(s, ref, err);
+        if (g.cur >= g.end) {
+            g.node = resume;
+            done = resume == kNone;
+        }
+    }
+    while (!done) done = group_step<ANY_HIT, BOUNDS, (int)G, TRI>(g, s, err, gl, gbase, gmask);
+    if (gl == 0) finish(item, g.slot, g.len, g.u, g.v);
 }
 
 }  // namespace gpugi

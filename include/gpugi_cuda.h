@@ -298,9 +298,10 @@ gpugi_status gpugi_trace_stats_device(gpugi_ctx* ctx, const gpugi_scene* scene,
  * (default): the same prefilter, then, on box hierarchies whose boxes nest
  * (every one that bvhmake or gpugi_scene_build makes), a walk over a four-wide
  * copy of the hierarchy, one lane per ray with leaves tested by eight lanes,
- * and on other scenes groups of 8 lanes that walk one ray together, testing a
- * window of consecutive preorder nodes or leaf slots per round; modes 4 and
- * 5: such groups of 4 and 16 lanes on every scene. All modes make the same
+ * and on other scenes a walk of the hierarchy itself, one lane per ray for long
+ * queues and for short ones groups of 8 lanes that walk one ray together,
+ * testing a window of consecutive preorder nodes or leaf slots per round;
+ * modes 4 and 5: such groups of 4 and 16 lanes on every scene. All modes make the same
  * decisions per ray as TraceRay and return identical results. blockSize
  * applies to mode 0. */
 gpugi_status gpugi_set_trace_config(gpugi_ctx* ctx, uint32_t mode, uint32_t blockSize);

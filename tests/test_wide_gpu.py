@@ -127,6 +127,21 @@ def test_queue_lengths(ctx, n):
     ds.close()
 
 
+@pytest.mark.parametrize("fit", ["ellipsoid", "obox"])
+@pytest.mark.parametrize("n", [3, 67000, 69000, 155649, 400001])
+def test_binary_queue_lengths(ctx, fit, n):
+    """Trees without a wide copy: both sides of the rule between groups and lanes (68,096 rays on 152
+    SMs), one full pass of the grid and refills."""
+    s = scenes.instanced_scene(seed=3, num_triangles=8000)
+    b = bvh.build_bvh(s["positions"], s["triangles"], method="sweep", fit=fit)
+    ds = ctx.upload_scene(b, s["positions"])
+    a, z = both_modes(ctx, ds, scenes.aimed_rays(n, s["positions"], seed=n, spread=0.8))
+    same(a, z)
+    rays = special_rays(s["positions"], 5, min(n, 80001))
+    same(*both_modes(ctx, ds, rays))
+    ds.close()
+
+
 @pytest.mark.parametrize("broken", ["not nested", "empty box", "nan box", "escape"])
 def test_trees_that_do_not_nest(ctx, broken):
     """Hierarchies the upload accepts but the wide copy must not be made of."""
