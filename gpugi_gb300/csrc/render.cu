@@ -191,13 +191,16 @@ GPUGI_D void persistent_walks(const DevScene& s, uint32_t n, unsigned long long*
     }
 }
 
-// Closest hits of the path queue. Queues shorter than groupBelow rays are
-// walked by 8-lane groups (group_walks: a short queue leaves lanes idle, and
-// groups shorten the longest walks); longer ones with one lane per ray (more
-// rays in flight; top nodes staged in shared memory). The choice depends on
-// the device-side count, so it costs no host round trip.
+// Closest hits of the path queue on scenes without a wide hierarchy. Queues
+// shorter than groupBelow rays are walked by 8-lane groups (group_walks: a
+// short queue leaves lanes idle, and groups shorten the longest walks); longer
+// ones with one lane per ray, by lane_walks, or by persistent_walks where the
+// scene's layout stages top nodes in shared memory. The choice depends on the
+// device-side count, so it costs no host round trip. Path tracing 512^2 x 8
+// (us, persistent_walks / lane_walks): room, ellipsoids 9,040 / 7,350, oriented
+// boxes 5,000 / 3,610; 30k instanced triangles 3,950 / 3,170 and 3,160 / 2,460.
 template <int BOUNDS>
-__global__ void __launch_bounds__(128) k_extend(RenderConst rc, PathSoA A, HitSoA H, int depth, uint32_t stage,
+__global__ void __launch_bounds__(128, 8) k_extend(RenderConst rc, PathSoA A, HitSoA H, int depth, uint32_t stage,
                                                 uint32_t groupBelow) {
     const uint32_t n = rc.cnt->path[depth];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&rc.cnt->rays[0], (unsigned long long)n);
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(128) k_extend(RenderConst rc, PathSoA A, HitSo
                                           H.u[i] = g.u;
                                           H.v[i] = g.v;
                                       });
-    } else {
+    } else if (stage) {
         persistent_walks<false, BOUNDS>(
             rc.s, n, &rc.cnt->extendWork[depth], rc.err, load,
             [&](uint32_t i, const WalkState& w) {
@@ -224,6 +227,15 @@ __global__ void __launch_bounds__(128) k_extend(RenderConst rc, PathSoA A, HitSo
                 H.v[i] = w.v;
             },
             stage);
+    } else {
+        __shared__ LaneShared sh;
+        lane_walks<false, BOUNDS, 0>(sh, rc.s, n, &rc.cnt->extendWork[depth], rc.err, load,
+                                     [&](uint32_t i, int32_t slot, float t, float u, float v) {
+                                         H.slot[i] = slot;
+                                         H.t[i] = t;
+                                         H.u[i] = u;
+                                         H.v[i] = v;
+                                     });
     }
 }
 
@@ -241,7 +253,7 @@ GPUGI_D void shadow_unoccluded(const RenderConst& rc, const ShadowSoA& Q, uint32
 }
 
 template <int BOUNDS>
-__global__ void __launch_bounds__(128) k_shadow(RenderConst rc, ShadowSoA Q, int depth, uint32_t stage,
+__global__ void __launch_bounds__(128, 8) k_shadow(RenderConst rc, ShadowSoA Q, int depth, uint32_t stage,
                                                 uint32_t groupBelow) {
     const uint32_t n = rc.cnt->shadow[depth];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&rc.cnt->rays[1], (unsigned long long)n);
@@ -255,13 +267,19 @@ __global__ void __launch_bounds__(128) k_shadow(RenderConst rc, ShadowSoA Q, int
                                      [&](uint64_t i, const GroupWalk& g) {
                                          if (g.slot < 0) shadow_unoccluded(rc, Q, (uint32_t)i);
                                      });
-    } else {
+    } else if (stage) {
         persistent_walks<true, BOUNDS>(
             rc.s, n, &rc.cnt->shadowWork[depth], rc.err, load,
             [&](uint32_t i, const WalkState& w) {
                 if (w.slot < 0) shadow_unoccluded(rc, Q, i);
             },
             stage);
+    } else {
+        __shared__ LaneShared sh;
+        lane_walks<true, BOUNDS, 0>(sh, rc.s, n, &rc.cnt->shadowWork[depth], rc.err, load,
+                                    [&](uint32_t i, int32_t slot, float, float, float) {
+                                        if (slot < 0) shadow_unoccluded(rc, Q, i);
+                                    });
     }
 }
 
@@ -2138,6 +2156,12 @@ static gpugi_status ensure_buffers_in(gpugi_ctx* ctx, RenderBuffers* rb, size_t 
     return GPUGI_OK;
 }
 
+// Queue length per block of the grid below which groups walk: twice the
+// lanes before persistent_walks, GPUGI_LANE_FROM before lane_walks.
+static uint32_t group_below(const Walkers& W) {
+    return W.LE.stage == 0 ? GPUGI_LANE_FROM : 128u * GPUGI_GROUP_BELOW_LANES;
+}
+
 static gpugi_status walkers_config(gpugi_ctx* ctx, const gpugi_scene* sc, Walkers& W) {
     W.bounds = (int)sc->dev.boundsKind;
     W.wide = sc->dev.wide && ctx->traceMode == 3;
@@ -2156,8 +2180,9 @@ static gpugi_status walkers_config(gpugi_ctx* ctx, const gpugi_scene* sc, Walker
     // workload: 0.5x, 2x, 8x, 64x the lanes gave PT 262 / 264.5 / 250 / 167 M
     // samples/s and the photon mapper 124 / 133 / 133 / 133)
     const bool group = ctx->traceMode >= 3;
-    W.groupBelowE = group ? W.LE.grid * 128u * GPUGI_GROUP_BELOW_LANES : 0u;
-    W.groupBelowS = group ? W.LS.grid * 128u * GPUGI_GROUP_BELOW_LANES : 0u;
+    const uint32_t below = group_below(W);
+    W.groupBelowE = group ? W.LE.grid * below : 0u;
+    W.groupBelowS = group ? W.LS.grid * below : 0u;
     return st;
 }
 
@@ -2793,8 +2818,8 @@ gpugi_status gpugi_render_nrc(gpugi_ctx* ctx, const gpugi_scene* sc, const gpugi
         const unsigned share = std::min(100u, 150u / (unsigned)nLanes);
         W.LE.grid = std::max(1u, W.LE.grid * share / 100u);
         W.LS.grid = std::max(1u, W.LS.grid * share / 100u);
-        if (W.groupBelowE) W.groupBelowE = W.LE.grid * 128u * GPUGI_GROUP_BELOW_LANES;
-        if (W.groupBelowS) W.groupBelowS = W.LS.grid * 128u * GPUGI_GROUP_BELOW_LANES;
+        if (W.groupBelowE) W.groupBelowE = W.LE.grid * group_below(W);
+        if (W.groupBelowS) W.groupBelowS = W.LS.grid * group_below(W);
     }
     int perSM = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, bpt ? (const void*)k_nrc_bpt_shade : (const void*)k_nrc_shade,
