@@ -71,5 +71,55 @@ GPUGI_D void encode(const Query& q, float3 boxMin, float3 boxInvExtent, __half* 
     while (k < kIn) out[k++] = __float2half(0.0f);
 }
 
+// The same encoding in 16-byte chunks of eight features (chunk c = features
+// [8 c, 8 c + 8)), for threads that share a query or store it chunk by chunk.
+struct EncodeInput {
+    float f[3];    // pi x position in the box; octave o of an axis is f 2^o, exactly
+    float sh[16];
+    float rest[7];
+};
+GPUGI_D EncodeInput encode_input(const Query& q, float3 boxMin, float3 boxInvExtent) {
+    EncodeInput e;
+    const float p[3] = {(q.pos.x - boxMin.x) * boxInvExtent.x, (q.pos.y - boxMin.y) * boxInvExtent.y,
+                        (q.pos.z - boxMin.z) * boxInvExtent.z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) e.f[d] = kPI_F * p[d];
+    const float x = q.dir.x, y = q.dir.y, z = q.dir.z;
+    const float xx = x * x, yy = y * y, zz = z * z;
+    const float sh[16] = {0.28209479f,
+                          -0.48860251f * y, 0.48860251f * z, -0.48860251f * x,
+                          1.09254843f * x * y, -1.09254843f * y * z, 0.31539157f * (3.0f * zz - 1.0f),
+                          -1.09254843f * x * z, 0.54627422f * (xx - yy),
+                          0.59004359f * y * (-3.0f * xx + yy), 2.89061144f * x * y * z,
+                          0.45704580f * y * (1.0f - 5.0f * zz), 0.37317633f * z * (5.0f * zz - 3.0f),
+                          0.45704580f * x * (1.0f - 5.0f * zz), 1.44530572f * z * (xx - yy),
+                          0.59004359f * x * (-xx + 3.0f * yy)};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) e.sh[i] = sh[i];
+    const float rest[7] = {q.normal.x, q.normal.y, q.normal.z, q.albedo.x, q.albedo.y, q.albedo.z, 1.0f};
+#pragma unroll
+    for (int i = 0; i < 7; ++i) e.rest[i] = rest[i];
+    return e;
+}
+template <int C>
+GPUGI_D uint4 encode_chunk(const EncodeInput& e) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = 8 * C + 2 * i;  // features k, k + 1
+        float a, b;
+        if (k < 36) {
+            sincosf(e.f[k / 12] * (float)(1 << (k % 12 / 2)), &a, &b);
+        } else {
+            auto get = [&](int j) { return j < 52 ? e.sh[j < 52 ? j - 36 : 0] : j < 59 ? e.rest[j >= 52 && j < 59 ? j - 52 : 0] : 0.0f; };
+            a = get(k);
+            b = get(k + 1);
+        }
+        __half2 h = __floats2half2_rn(a, b);
+        w[i] = *reinterpret_cast<uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 }  // namespace nrc
 }  // namespace gpugi

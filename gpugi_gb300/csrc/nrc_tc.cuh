@@ -64,10 +64,11 @@ GPUGI_D uint64_t globaltimer_ns() {
 }
 // Wait for the phase `parity` of an mbarrier, at most limitNs nanoseconds
 // of the global timer (and at most 2^24 polls, should the timer not
-// advance); false when the wait ran out.
+// advance); false when the wait ran out. The timer is first read after 256
+// polls: a wait that ends sooner (every one but a lost one) never reads it.
 GPUGI_D bool bar_wait(uint64_t* bar, uint32_t parity, uint64_t limitNs) {
     const uint32_t a = smem_addr(bar);
-    const uint64_t t0 = globaltimer_ns();
+    uint64_t t0 = 0;
     for (uint32_t it = 0; it < (1u << 24); ++it) {
         uint32_t done;
         asm volatile(
@@ -76,7 +77,11 @@ GPUGI_D bool bar_wait(uint64_t* bar, uint32_t parity, uint64_t limitNs) {
             : "r"(a), "r"(parity)
             : "memory");
         if (done) return true;
-        if ((it & 255u) == 255u && globaltimer_ns() - t0 > limitNs) return false;
+        if ((it & 255u) == 255u) {
+            const uint64_t now = globaltimer_ns();
+            if (it == 255u) t0 = now;
+            else if (now - t0 > limitNs) return false;
+        }
     }
     return false;
 }
@@ -103,6 +108,16 @@ GPUGI_D void ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+GPUGI_D void ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
 GPUGI_D void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
