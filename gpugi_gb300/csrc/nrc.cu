@@ -772,38 +772,39 @@ __global__ void __launch_bounds__(256, 1) k_nrc_train_tc(const float* __restrict
 }
 
 // ----------------------------------------------- tcgen05 inference kernel
-// Two warpgroups per CTA, each running its own chain of 128-query tiles:
-// thread t of a warpgroup owns query t of the tile (TMEM lane t), one
+// tci::kChains warpgroups per CTA, each running its own chain of 128-query
+// tiles: thread t of a warpgroup owns query t of the tile (TMEM lane t), one
 // thread per warpgroup issues the five layers' MMAs (D = X W_l) into the
 // warpgroup's 64 TMEM columns and its mbarrier tracks them; between layers
 // the warpgroup turns D into the next layer's fp16 input (ReLU) in its own
 // 16 KB X buffer. The weights (the moving average, [in][out] as the
-// training weights) are staged once per CTA. 3 CTAs fit an SM (66 KB of
-// shared memory, 128 TMEM columns each), so six chains overlap their
-// latencies.
+// training weights) are staged once per CTA. Bound by the chain's latency and
+// by issue slots (~1,400 instructions per query, 800 of them the 18 sines and
+// cosines): 2 CTAs of four chains fill an SM's TMEM (512 columns) and
+// registers (64 x 1,024), a tile's records are fetched during the tile before
+// it, as 16-B loads where the array allows it.
 namespace tci {
 constexpr uint32_t kXSG = 8 * 128, kXBytes = 16 * kXSG;
 constexpr uint32_t kWBytes = tcl::kWBytes;
-constexpr uint32_t kSmem = kWBytes + 2 * kXBytes + 1024;
+// chains per CTA x CTAs per SM, a lookup of 921,600 queries through the public call: 2 x 3 106.6 us,
+// 3 x 2 104.7, 1 x 4 111.0, 2 x 4 115.0, 4 x 2 102.7 (109.4 before, 2 x 3 without the early fetch)
+constexpr uint32_t kChains = 4, kCtas = 2;
+constexpr uint32_t kCols = 64 * kChains;  // a power of two
+constexpr uint32_t kSmem = kWBytes + kChains * kXBytes + 1024;
 }  // namespace tci
 
 // A barrier of the warpgroup's 128 threads that also ORs a flag over them.
 GPUGI_D bool wg_any(int wg, bool v) {
     uint32_t r;
-    if (wg == 0)
-        asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, 1, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(r)
-                     : "r"((uint32_t)v)
-                     : "memory");
-    else
-        asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, 2, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(r)
-                     : "r"((uint32_t)v)
-                     : "memory");
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, %2, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(r)
+                 : "r"((uint32_t)v), "r"(wg + 1)
+                 : "memory");
     return r != 0;
 }
 
-__global__ void __launch_bounds__(256) k_nrc_infer_tc(const float* __restrict__ queries, uint64_t n,
+template <bool VEC>
+__global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc(const float* __restrict__ queries, uint64_t n,
                                                       const uint32_t* __restrict__ count,
                                                       const __half* __restrict__ wInfT, float3 boxMin, float3 boxInv,
                                                       float* __restrict__ out, uint32_t* errWord, uint64_t waitNs,
@@ -813,7 +814,7 @@ __global__ void __launch_bounds__(256) k_nrc_infer_tc(const float* __restrict__ 
     if (count) n = min(n, (uint64_t)*count);
     extern __shared__ uint8_t smemRaw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t bars[2];
+    __shared__ uint64_t bars[tci::kChains];
     __shared__ uint32_t tmemBase;
     const int t = threadIdx.x, wg = t >> 7, lt = t & 127, warp = t >> 5;
     for (int l = 0; l < kLayers; ++l) {
@@ -825,10 +826,9 @@ __global__ void __launch_bounds__(256) k_nrc_infer_tc(const float* __restrict__ 
         }
     }
     if (t == 0) {
-        bar_init(&bars[0], 1);
-        bar_init(&bars[1], 1);
+        for (uint32_t k = 0; k < tci::kChains; ++k) bar_init(&bars[k], 1);
     }
-    if (warp == 0) tmem_alloc(&tmemBase, 128);
+    if (warp == 0) tmem_alloc(&tmemBase, tci::kCols);
     fence_smem();
     fence_before();
     __syncthreads();
@@ -842,26 +842,46 @@ __global__ void __launch_bounds__(256) k_nrc_infer_tc(const float* __restrict__ 
     uint32_t parity = 0;
     bool failed = false;
     const uint64_t tiles = (n + 127) / 128;
-    for (uint64_t tile = 2 * (uint64_t)blockIdx.x + wg; tile < tiles && !failed; tile += 2 * (uint64_t)gridDim.x) {
+    float4 p[3];  // the thread's record of the next tile
+    auto fetch = [&](uint64_t tile) {
         const uint64_t row = tile * 128 + (uint64_t)lt;
-        {
-            __align__(16) __half enc[kIn];
-            if (row < n) {
-                const float* p = queries + 12 * row;
-                Query q;
-                q.pos = make_float3(p[0], p[1], p[2]);
-                q.dir = make_float3(p[3], p[4], p[5]);
-                q.normal = make_float3(p[6], p[7], p[8]);
-                q.albedo = make_float3(p[9], p[10], p[11]);
-                encode(q, boxMin, boxInv, enc);
-            } else {
+        if (VEC) {
+            const float4* q = reinterpret_cast<const float4*>(queries) + 3 * row;
 #pragma unroll
-                for (int k = 0; k < kIn; ++k) enc[k] = __float2half(0.0f);
-            }
+            for (int k = 0; k < 3; ++k) p[k] = row < n ? __ldg(q + k) : make_float4(0, 0, 0, 0);
+        } else {
+            const float* q = queries + 12 * row;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<uint4*>(xRow + j * 128) = *reinterpret_cast<const uint4*>(enc + 8 * j);
+            for (int k = 0; k < 3; ++k)
+                p[k] = row < n ? make_float4(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]) : make_float4(0, 0, 0, 0);
         }
+    };
+    const uint64_t stride = tci::kChains * (uint64_t)gridDim.x;
+    uint64_t tile = tci::kChains * (uint64_t)blockIdx.x + wg;
+    fetch(tile);
+    for (; tile < tiles && !failed; tile += stride) {
+        const uint64_t row = tile * 128 + (uint64_t)lt;
+        if (row < n) {
+            Query q;
+            q.pos = make_float3(p[0].x, p[0].y, p[0].z);
+            q.dir = make_float3(p[0].w, p[1].x, p[1].y);
+            q.normal = make_float3(p[1].z, p[1].w, p[2].x);
+            q.albedo = make_float3(p[2].y, p[2].z, p[2].w);
+            const EncodeInput e = encode_input(q, boxMin, boxInv);
+            uint4* x = reinterpret_cast<uint4*>(xRow);
+            x[0] = encode_chunk<0>(e);
+            x[8] = encode_chunk<1>(e);
+            x[16] = encode_chunk<2>(e);
+            x[24] = encode_chunk<3>(e);
+            x[32] = encode_chunk<4>(e);
+            x[40] = encode_chunk<5>(e);
+            x[48] = encode_chunk<6>(e);
+            x[56] = encode_chunk<7>(e);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(xRow + j * 128) = make_uint4(0, 0, 0, 0);
+        }
+        fetch(tile + stride);
         for (int l = 0; l < kLayers; ++l) {
             // the layer's barrier also agrees on a timeout: a warpgroup
             // leaves together, never with some threads waiting here
@@ -912,7 +932,7 @@ __global__ void __launch_bounds__(256) k_nrc_infer_tc(const float* __restrict__ 
     fence_before();
     __syncthreads();
     fence_after();
-    if (warp == 0) tmem_free(tmemBase, 128);
+    if (warp == 0) tmem_free(tmemBase, tci::kCols);
 }
 
 // grad[i] = sum over the CTAs' partial sums, in a fixed order
@@ -986,17 +1006,20 @@ gpugi_status gpugi::nrc_infer_counted(gpugi_ctx* ctx, const gpugi_nrc* nn, const
                                       const uint32_t* count, float* out) {
     if (n == 0) return GPUGI_OK;
     if (nn->kernels == GPUGI_NRC_KERNELS_TCGEN05) {
+        auto k = ((uintptr_t)queries & 15u) == 0 ? &k_nrc_infer_tc<true> : &k_nrc_infer_tc<false>;
         static bool tcAttr = false;
         if (!tcAttr) {
-            GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(k_nrc_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(k_nrc_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)tci::kSmem));
+            GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(k_nrc_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)tci::kSmem));
             tcAttr = true;
         }
         const uint64_t tiles = (n + 127) / 128;
-        const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->numSMs * 3, (tiles + 1) / 2);
-        k_nrc_infer_tc<<<(unsigned)grid, 256, tci::kSmem, ctx->stream>>>(queries, n, count, nn->wInfT, nn->boxMin,
-                                                                         nn->boxInv, out, ctx->errWord, nn->waitNs,
-                                                                         nn->stall);
+        const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->numSMs * tci::kCtas, (tiles + tci::kChains - 1) / tci::kChains);
+        k<<<(unsigned)grid, 128 * tci::kChains, tci::kSmem, ctx->stream>>>(queries, n, count, nn->wInfT, nn->boxMin,
+                                                                           nn->boxInv, out, ctx->errWord, nn->waitNs,
+                                                                           nn->stall);
         GPUGI_CUDA_TRY(ctx, cudaGetLastError());
         return GPUGI_OK;
     }

@@ -192,3 +192,31 @@ def test_training_learns_a_smooth_field(cuda_ctx):
     assert loss < 0.1 * first, (first, loss)
     assert rel < 0.1, rel
     c.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 512, 513, 155648, 155649, 160001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_inference_sizes_and_alignment(n, shift):
+    """The tcgen05 lookups against the mma.sync ones: part tiles, part CTAs, one tile per chain of the
+    full grid (8 x 152 tiles) and one more, records on 16-B and on 4-B boundaries. The same fp16
+    weights, encodings and activations, f32 sums in another order: a sum of 64 terms differs by at
+    most 64 * 2^-24 of its absolute terms, which can move an activation by one fp16 step (2^-10
+    relative) in each of the four hidden layers."""
+    import torch
+    from gpugi_gb300 import cuda, nrc
+    ctx = cuda.Context(0)
+    rng = np.random.default_rng(n)
+    q = rng.uniform(-1, 1, (n, 12)).astype(np.float32)
+    buf = torch.zeros(12 * n + 4, device="cuda")
+    view = buf[shift:shift + 12 * n].view(n, 12)
+    view.copy_(torch.from_numpy(q))
+    c = nrc.RadianceCache(ctx, (-1, -1, -1), (1, 1, 1), seed=3)
+    out = {}
+    for k in nrc.KERNELS:
+        c.set_kernels(k)
+        out[k] = c.infer(view).cpu().numpy()
+    scale = max(1.0, float(np.abs(out["mma_sync"]).max()))
+    assert np.abs(out["tcgen05"] - out["mma_sync"]).max() <= 4 * 8 * 2.0 ** -10 * scale
+    assert ctx.device_error_bits() == 0
+    c.close()
+    ctx.close()
