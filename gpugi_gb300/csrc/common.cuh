@@ -110,12 +110,13 @@ constexpr uint32_t LEAF_BLOCK_MASK = 0x01FFFFFFu;
 constexpr uint32_t LEAF_COUNT_SHIFT = 25;
 constexpr uint32_t LEAF_COUNT_MASK = 0x3Fu;
 
-// Wide hierarchy (wide.cu): reference of an unused child; entries of a walk's
-// stack (kWideShared of them in shared memory, the rest in local memory).
-// Walks of the measured scenes hold at most 10; a walk that expands waiting
-// nodes early does so within the shared part only, so kWideShared + 3 per
-// wide level bounds the stack.
+// Wide hierarchy (wide.cu): reference of an unused child; entries of a lane's
+// stack (kWideShared of them in shared memory, the rest in local memory; walks
+// of the measured scenes hold at most 10): three per wide level at most. The
+// stack of a ray that a whole warp walks takes in waiting nodes early only
+// while it holds at most 32 entries, which then become 56 at most, and three
+// per level above those: 56 + kWideStack and the current reference.
 constexpr uint32_t kWideEmpty = 0xFFFFFFFFu;
-constexpr uint32_t kWideShared = 12, kWideStack = 84;
+constexpr uint32_t kWideShared = 8, kWideStack = 72, kWarpStack = 136;
 
 }  // namespace gpugi

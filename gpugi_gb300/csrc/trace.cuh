@@ -626,29 +626,24 @@ GPUGI_D void group_walks_multi(uint64_t n, unsigned long long* work, uint32_t* e
 // of waiting children cost 2-8 %.
 // Measured against the binary walkers: 3M any-hit rays in the terrain
 // 2.19 to 0.85 ms, path tracing the room at 512^2 x 16 samples 15.98 to
-// 9.5 ms, light tracing 9.16 to 5.4 ms, 1,000 rays (one per warp, the last
-// stage alone) 43 to 27 us.
+// 9.3 ms, light tracing 9.16 to 5.3 ms, 1,000 rays (a warp each) 43 to 18 us, a
+// 320 x 180 frame 1.03 to 0.63 ms (0.92 with eight lanes per ray at the end).
 GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
 
-// Lanes of a warp step through nodes together until this many leaves wait or
-// fewer than so many lanes have a node left (leaf lanes 4 / 8 / 12: 10.09 /
-// 9.94 / 9.94 ms for the path-traced room; node lanes 4-12: the same), fetch
-// new rays when at least so many lanes are free (1 / 8 / 12 / 16: 1.04 /
-// 0.98 / 0.97 / 0.99 of the terrain's time), and hand the rays over to eight
-// lanes each when no more than two are left (0 / 2 / 4: 1.06 / 0.96 / 0.97 ms
-// for a 320 x 180 frame of one sample, whose queues end in long single walks).
-#ifndef GPUGI_WIDE_NODE_LANES
-#define GPUGI_WIDE_NODE_LANES 8
-#endif
-#ifndef GPUGI_WIDE_LEAF_LANES
-#define GPUGI_WIDE_LEAF_LANES 8
-#endif
-#ifndef GPUGI_WIDE_REFILL
-#define GPUGI_WIDE_REFILL 12
-#endif
-#ifndef GPUGI_WIDE_GROUP_AT
-#define GPUGI_WIDE_GROUP_AT 2
-#endif
+// Lanes of a warp step through nodes together until kWideLeaves leaves wait or
+// fewer than kWideNodes lanes have a node left (leaves 4 / 8 / 12: 10.09 / 9.94
+// / 9.94 ms for the path-traced room; node lanes 4-12: the same), fetch new
+// rays when at least kWideRefill lanes are free (1 / 8 / 12 / 16: 1.04 / 0.98 /
+// 0.97 / 0.99 of the terrain's time), and hand their rays over, one after
+// another, to the whole warp when no more than kWideWarpAt are left: the long
+// single walks that a queue ends with then take a few rounds (at 1 / 2 / 4 / 6
+// / 10 rays: 748 / 691 / 664 / 664 / 678 us for a 320 x 180 frame of one sample,
+// 137 / 129 / 120 / 118 / 123 for 66k rays in the icosphere). Queues of at most
+// kWideSolo rays per warp are walked that way from the start (1 / 4 / 8 / 16 /
+// 32: 664 / 655 / 623 / 616 / 617 us for the frame; 119 / 127 us at 8 / 16 for
+// the icosphere's 66k).
+constexpr int kWideLeaves = 8, kWideNodes = 8, kWideRefill = 12, kWideWarpAt = 5;
+constexpr uint32_t kWideSolo = 8;
 // Resident blocks per SM that the wide walkers are compiled for (64
 // registers; 7 / 8 / 9 blocks: 9.94 / 9.60 / 9.63 ms for the path-traced room).
 #ifndef GPUGI_WIDE_MIN_BLOCKS
@@ -658,6 +653,7 @@ GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfini
 struct WideShared {
     uint2 e[kWideShared][128];  // stack entries {reference, entry distance}, a column per ray
     float4 ray[2][128];         // {origin, d.x}, {d.y, d.z, -, -}
+    uint2 w[4][kWarpStack];     // stack of the ray a whole warp walks
 };
 
 // Valid slots of a leaf word (checked builds: none where they pass the end).
@@ -836,21 +832,23 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
     const unsigned C = n >= 32 * (uint64_t)warps ? 32u : ((uint32_t)n + warps - 1) / warps;
     const uint64_t first = (uint64_t)warps * C;
     bool more = n > first;
-    {
-        const uint64_t i = ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * C + lane;
+    const uint64_t warp = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const bool solo = n <= (uint64_t)warps * kWideSolo;
+    if (!solo) {
+        const uint64_t i = warp * C + lane;
         if (lane < C && i < n) begin((uint32_t)i);
     }
     // ---- a ray per lane
-    while (true) {
+    while (!solo) {
         const unsigned act = __ballot_sync(0xffffffffu, active);
-        if (more && __popc(act) <= 32 - GPUGI_WIDE_REFILL) {
+        if (more && __popc(act) <= 32 - kWideRefill) {
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(work, (unsigned long long)__popc(~act));
             base = first + __shfl_sync(0xffffffffu, base, 0);
             more = base + __popc(~act) < n;
             base += (unsigned)__popc(~act & ((1u << lane) - 1u));
             if (!active && base < n) begin((uint32_t)base);
-        } else if (!more && __popc(act) <= GPUGI_WIDE_GROUP_AT) {
+        } else if (!more && __popc(act) <= kWideWarpAt) {
             break;
         }
         // nodes
@@ -932,7 +930,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
             }
             const unsigned nodes = __ballot_sync(0xffffffffu, active && !(ref & LEAF_FLAG));
             const unsigned leaves = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
-            if (__popc(leaves) >= GPUGI_WIDE_LEAF_LANES || __popc(nodes) < GPUGI_WIDE_NODE_LANES || !nodes) break;
+            if (__popc(leaves) >= kWideLeaves || __popc(nodes) < kWideNodes || !nodes) break;
         }
         // leaves: four at a time, eight lanes each
         unsigned todo = __ballot_sync(0xffffffffu, active && (ref & LEAF_FLAG));
@@ -951,141 +949,184 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                 }
             });
     }
-    // ---- eight lanes per ray
-    constexpr unsigned G = 8;
-    const unsigned gl = lane & (G - 1), gbase = lane & ~(G - 1), gmask = 0xffu << gbase;
-    {
-        unsigned act = __ballot_sync(0xffffffffu, active);
-        if (!act) return;
-        for (unsigned g = 0; g < lane / G; ++g) act &= act - 1;
-        const unsigned src = act ? (unsigned)(__ffs(act) - 1) : 0u;
-        auto get = [&](float x) { return __shfl_sync(0xffffffffu, x, src); };
-        auto get2 = [&](float2 x) { const float y = get(x.x); return make_float2(y, y); };
-        auto geti = [&](uint32_t x) { return __shfl_sync(0xffffffffu, x, src); };
-        nox = get2(nox), noy = get2(noy), noz = get2(noz);
-        ivx = get2(ivx), ivy = get2(ivy), ivz = get2(ivz);
-        len = get(len);
-        u = get(u);
-        v = get(v);
-        slot = (int32_t)geti((uint32_t)slot);
-        budget = geti(budget);
-        ref = geti(ref);
-        const uint32_t deepest = __reduce_max_sync(0xffffffffu, active && !seq ? sp : 0u);
-        sp = geti(sp);
-        item = geti(item);
-        axis = geti(axis) != 0;
-        seq = geti(seq) != 0;
-        col = (threadIdx.x & ~31u) + src;
-        for (uint32_t k = kWideShared; k < deepest; ++k) {
-            const uint2 e = deep[k - kWideShared];
-            deep[k - kWideShared] = make_uint2(geti(e.x), geti(e.y));
-        }
-        __syncwarp();
-        if (MULTI) {
-            own = shfl_scene(0xffffffffu, src);
-            wide = reinterpret_cast<const char*>(own->wide);
-        }
-        if (!act) return;
-    }
-    const float4 r0 = sh.ray[0][col], r1 = sh.ray[1][col];
-    const float3 o = make_float3(r0.x, r0.y, r0.z), d = make_float3(r0.w, r1.x, r1.y);
-    WtRay wt = {};
-    if (TRI) wt = wt_setup(d);
+    // ---- a warp per ray
+    // Every lane holds the ray; the stack is the warp's. A node round expands up to eight entries from
+    // the top (waiting nodes early, waiting leaves stay), a leaf round tests up to four leading leaves
+    // and resolves them in order.
+    uint2* const ws = sh.w[threadIdx.x >> 5];
+    uint64_t next = warp;
     while (true) {
-        if (ref & LEAF_FLAG) {
-            const uint32_t block = ref & LEAF_BLOCK_MASK, k0 = block * own->leafSize;
-            const uint32_t cnt = leaf_slots(*own, ref, err);
-            bool done = false;
-            for (uint32_t off = 0; off < cnt; off += G) {
+        unsigned src = 0;
+        if (solo) {
+            if (next >= n) break;
+            if (lane == 0) begin((uint32_t)next);
+            __syncwarp();
+        } else {
+            const unsigned act = __ballot_sync(0xffffffffu, active);
+            if (!act) break;
+            src = (unsigned)(__ffs(act) - 1);
+        }
+        auto get = [&](float x) { return __shfl_sync(0xffffffffu, x, src); };
+        auto geti = [&](uint32_t x) { return __shfl_sync(0xffffffffu, x, src); };
+        const unsigned scol = (threadIdx.x & ~31u) + src;
+        const float4 r0 = sh.ray[0][scol], r1 = sh.ray[1][scol];
+        const float3 o = make_float3(r0.x, r0.y, r0.z), d = make_float3(r0.w, r1.x, r1.y);
+        const float3 wi = make_float3(get(ivx.x), get(ivy.x), get(ivz.x));
+        WtRay wt = {};
+        if (TRI) wt = wt_setup(d);
+        float wlen = get(len), wu = get(u), wv = get(v);
+        int32_t wslot = (int32_t)geti((uint32_t)slot);
+        const uint32_t witem = geti(item);
+        uint32_t wref = geti(ref), wsp = geti(sp), wbudget = geti(budget);
+        const bool waxis = geti(axis) != 0;
+        bool wseq = geti(seq) != 0;
+        const DevScene* const ws_scene = MULTI ? shfl_scene(0xffffffffu, src) : own;
+        const DevScene& s = *ws_scene;
+        const float4* const tris = TRI ? s.wtris : s.tris;
+        const char* const wwide = reinterpret_cast<const char*>(s.wide);
+        // the ray's stack, with the reference it holds on top (a sequential walk keeps its escape in wsp)
+        if (!wseq) {
+            for (uint32_t k = lane; k < min(wsp, kWideShared); k += 32) ws[k] = sh.e[k][scol];
+            for (uint32_t k = kWideShared; k < wsp; ++k) {
+                const uint2 e = deep[k - kWideShared];
+                const uint2 x = make_uint2(geti(e.x), geti(e.y));
+                if (lane == 0) ws[k] = x;
+            }
+            if (lane == 0) ws[wsp] = make_uint2(wref, 0u);  // firstHit already compared with this rayLength
+            ++wsp;
+            __syncwarp();
+        }
+        // `leaves` leading leaves, lane group g's word lref with entry distance lf; true when any hit is done
+        auto test_leaves = [&](uint32_t lref, float lf, unsigned leaves) {
+            const unsigned g = lane >> 3, gl = lane & 7u;
+            const uint32_t k0 = g < leaves ? (lref & LEAF_BLOCK_MASK) * s.leafSize : 0u;
+            const uint32_t cnt = g < leaves ? leaf_slots(s, lref, err) : 0u;
+            for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
                 float h = 0.0f, hu = 0.0f, hv = 0.0f;
                 bool ok = false;
-                if (off + gl < cnt) {
-                    const float4* rec = tris_of(*own) + 3 * (size_t)(k0 + off + gl);
+                if (off < cnt) {
+                    const float4* rec = tris + 3 * (size_t)(k0 + off);
                     const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
                     ok = TRI ? intersect_triangle_wt_v(o, wt, a, b, c, h, hu, hv)
                              : intersect_triangle_v(o, d, a, b, c, h, hu, hv);
-                    ok = ok && h < len;
+                    ok = ok && h < wlen && lf <= wlen;
                 }
-                if (__any_sync(gmask, ok)) {
-                    if (ANY_HIT) {
-                        slot = 0;
-                        done = true;
-                        break;
+                if (!__any_sync(0xffffffffu, ok)) continue;
+                if (ANY_HIT) {
+                    wslot = 0;
+                    return true;
+                }
+                const uint32_t hb = ok ? __float_as_uint(h) : 0x7fffffffu;
+                uint32_t mn = min(hb, __shfl_xor_sync(0xffffffffu, hb, 4));
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+                const unsigned tie = __ballot_sync(0xffffffffu, ok && hb == mn);
+                for (unsigned k = 0; k < leaves; ++k) {  // in order: each with the rayLength the ones before left
+                    const unsigned gm = tie >> (8 * k) & 0xffu;
+                    if (!gm) continue;
+                    const unsigned win = 8 * k + (unsigned)__ffs(gm) - 1;
+                    const float kf = __shfl_sync(0xffffffffu, lf, win), kh = __shfl_sync(0xffffffffu, h, win);
+                    if (kf <= wlen && kh < wlen) {
+                        wlen = kh;
+                        wu = __shfl_sync(0xffffffffu, hu, win);
+                        wv = __shfl_sync(0xffffffffu, hv, win);
+                        wslot = (int32_t)__shfl_sync(0xffffffffu, k0 + off, win);
                     }
-                    const uint32_t hb = __reduce_min_sync(gmask, ok ? __float_as_uint(h) : 0x7fffffffu);
-                    const unsigned tie = __ballot_sync(gmask, ok && __float_as_uint(h) == hb);
-                    const unsigned win = (unsigned)(__ffs(tie) - 1);
-                    u = __shfl_sync(gmask, hu, win);
-                    v = __shfl_sync(gmask, hv, win);
-                    slot = (int32_t)(k0 + off + (win - gbase));
-                    len = __uint_as_float(hb);
                 }
             }
-            ref = kNone;
-            if (done) break;
-        } else if (guard(seq ? own->numNodes : own->numWide)) {
-        } else if (!seq) {
-            // lanes 0-3: the children of `ref`; lanes 4-7: those of the next pending child if that
-            // is a node too (it is expanded early; its children are compared with rayLength when
-            // they are taken), so that a round tests two nodes
-            uint32_t mine = gl < 4 ? ref : kNone;
-            if (sp > 0 && sp <= kWideShared - 6) {
-                const uint2 e = sh.e[sp - 1][col];
-                if (!(e.x & LEAF_FLAG)) {
-                    --sp;
-                    if (gl >= 4 && (ANY_HIT || __uint_as_float(e.y) <= len)) mine = e.x;
+            return false;
+        };
+        while (true) {
+            if (wseq) {  // the binary tree, one node at a time
+                if (wref & LEAF_FLAG) {
+                    if (test_leaves(wref, 0.0f, 1)) break;
+                    if (wsp == 0) break;
+                    wref = wsp;
+                    wsp = 0;
+                    continue;
                 }
-            }
-            bool hit = false, restart = false;
-            float f = 0.0f;
-            uint32_t r = kNone;
-            if (mine != kNone) {
-                const float* nd = reinterpret_cast<const float*>(wide + 128 * (size_t)mine) + (gl & 3u);
-                const float4 lo = make_float4(__ldg(nd), __ldg(nd + 8), __ldg(nd + 16), 0.0f);
-                const float4 hi = make_float4(__ldg(nd + 4), __ldg(nd + 12), __ldg(nd + 20), 0.0f);
-                r = __float_as_uint(__ldg(nd + 24));
-                hit = intersect_box<TRI != 0>(o, invdir(), lo, hi, f) && f <= len && r != kWideEmpty;
-                if (TRI == 0 && axis) restart = hit && flat(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z));
-            }
-            if (TRI == 0 && axis && __any_sync(gmask, restart)) {
-                begin(item);
-                seq = true;
+                if (wbudget-- == 0 || (kChecked && wref >= s.numNodes)) {
+                    raise_error(err, kChecked && wref >= s.numNodes ? DEVERR_BOUNDS : DEVERR_TRAVERSAL_CAP);
+                    break;
+                }
+                const float4 a = __ldg(s.nodes + 2 * (size_t)wref), b = __ldg(s.nodes + 2 * (size_t)wref + 1);
+                float f;
+                const bool hit = intersect_box<TRI != 0>(o, wi, a, b, f) && f <= wlen;
+                const uint32_t child = __float_as_uint(a.w), esc = __float_as_uint(b.w);
+                if (hit && (child & LEAF_FLAG)) wsp = esc;
+                wref = hit ? child : esc;
+                if (!hit && esc == 0) break;
                 continue;
             }
-            const unsigned m = __ballot_sync(gmask, hit);
-            ref = kNone;
-            if (m) {
-                const unsigned lo = (unsigned)(__ffs(m) - 1);
-                ref = __shfl_sync(gmask, r, lo);
-                const unsigned pushes = (unsigned)__popc(m) - 1;
-                if (pushes) {
-                    if (sp + pushes <= kWideShared) {
-                        if (hit && lane != lo)
-                            sh.e[sp + __popc(m >> lane) - 1][col] = make_uint2(r, __float_as_uint(f));
-                        sp += pushes;
-                    } else {
-                        for (unsigned rest = m & (m - 1); rest;) {
-                            const unsigned top = 31u - (unsigned)__clz(rest);
-                            rest &= ~(1u << top);
-                            const uint2 e = make_uint2(__shfl_sync(gmask, r, top),
-                                                       __float_as_uint(__shfl_sync(gmask, f, top)));
-                            if (sp < kWideShared) sh.e[sp][col] = e;
-                            else deep[sp - kWideShared] = e;
-                            ++sp;
-                        }
-                    }
-                    __syncwarp(gmask);
-                }
+            if (wsp == 0) break;
+            if (ws[wsp - 1].x & LEAF_FLAG) {
+                const unsigned g = lane >> 3;
+                uint2 e = make_uint2(0, 0);
+                if (g < wsp) e = ws[wsp - 1 - g];
+                const bool leaf = (e.x & LEAF_FLAG) != 0, large = (e.x >> LEAF_COUNT_SHIFT & LEAF_COUNT_MASK) > 8;
+                const unsigned lm = __ballot_sync(0xffffffffu, leaf);
+                // leading leaves; one at a time where a block takes more than one pass of eight lanes
+                const unsigned lead = __any_sync(0xffffffffu, leaf && large) ? 1u
+                                      : lm == 0xffffffffu ? 4u : ((unsigned)__ffs(~lm) - 1) / 8;
+                wsp -= lead;
+                if (test_leaves(e.x, __uint_as_float(e.y), lead)) break;
                 continue;
             }
-        } else {
-            seq_node();
-            if (ref != kNone) continue;
+            if (wbudget == 0) {
+                raise_error(err, DEVERR_TRAVERSAL_CAP);
+                break;
+            }
+            // several entries only while the stack keeps room for the depth first bound above them
+            const uint32_t m = wsp <= 32 ? min(wsp, 8u) : 1u;
+            const uint32_t k = lane >> 2;
+            uint2 e = make_uint2(kNone, 0u);
+            if (k < m) e = ws[wsp - 1 - k];
+            bool hit = k < m && (ANY_HIT || __uint_as_float(e.y) <= wlen), restart = false;
+            float f = __uint_as_float(e.y);
+            uint32_t r = e.x;
+            if (e.x & LEAF_FLAG) {
+                hit = hit && (lane & 3u) == 0;  // a waiting leaf stays
+            } else if (hit) {
+                if (kChecked && e.x >= s.numWide) {
+                    raise_error(err, DEVERR_BOUNDS);
+                    hit = false;
+                } else {
+                    const float* nd = reinterpret_cast<const float*>(wwide + 128 * (size_t)e.x) + (lane & 3u);
+                    const float4 lo = make_float4(__ldg(nd), __ldg(nd + 8), __ldg(nd + 16), 0.0f);
+                    const float4 hi = make_float4(__ldg(nd + 4), __ldg(nd + 12), __ldg(nd + 20), 0.0f);
+                    r = __float_as_uint(__ldg(nd + 24));
+                    hit = intersect_box<TRI != 0>(o, wi, lo, hi, f) && f <= wlen && r != kWideEmpty;
+                    if (TRI == 0 && waxis)
+                        restart = hit && ((isinf(wi.x) && lo.x == o.x && hi.x == o.x) ||
+                                          (isinf(wi.y) && lo.y == o.y && hi.y == o.y) ||
+                                          (isinf(wi.z) && lo.z == o.z && hi.z == o.z));
+                }
+            }
+            if (TRI == 0 && waxis && __any_sync(0xffffffffu, restart)) {
+                float3 x, y;
+                load(witem, x, y, wlen);
+                wslot = -1;
+                wu = wv = 0.0f;
+                wseq = true;
+                wref = wsp = 0;
+                wbudget = s.numNodes;
+                continue;
+            }
+            --wbudget;  // every round expands a node
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            __syncwarp();
+            if (hit) ws[wsp - m + __popc(hits >> lane) - 1] = make_uint2(r, __float_as_uint(f));
+            wsp += (uint32_t)__popc(hits) - m;
+            __syncwarp();
         }
-        pop();
-        if (ref == kNone) break;
+        if (lane == 0) finish(witem, wslot, wlen, wu, wv);
+        __syncwarp();
+        if (lane == src) active = false;
+        if (solo) {
+            if (lane == 0) next = warps + atomicAdd(work, 1ull);
+            next = __shfl_sync(0xffffffffu, next, 0);
+        }
     }
-    if (gl == 0) finish(item, slot, len, u, v);
 }
 
 // ----------------------------------------------------------------- lane walk

@@ -175,7 +175,7 @@ gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc) {
     GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got + 2, index + n, 4, cudaMemcpyDeviceToHost, st));
     GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     // a walk's stack holds at most three entries per wide level, and its node offsets are 32-bit bytes
-    const bool fits = 3 * (~got[1] / 2 + 1) + kWideShared <= kWideStack && got[2] < (1u << 25);
+    const bool fits = 3 * (~got[1] / 2 + 1) <= kWideStack && got[2] < (1u << 25);
     if (got[0] == 0 || !fits || got[2] == 0 || got[2] > count) return GPUGI_OK;
     sc->wide = sc->dev.wide = wide;
     sc->dev.numWide = got[2];
