@@ -857,7 +857,8 @@ __global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc
         }
     };
     const uint64_t stride = tci::kChains * (uint64_t)gridDim.x;
-    uint64_t tile = tci::kChains * (uint64_t)blockIdx.x + wg;
+    // few tiles: one chain of each CTA before the second of any
+    uint64_t tile = (uint64_t)wg * gridDim.x + blockIdx.x;
     fetch(tile);
     for (; tile < tiles && !failed; tile += stride) {
         const uint64_t row = tile * 128 + (uint64_t)lt;
@@ -1016,7 +1017,7 @@ gpugi_status gpugi::nrc_infer_counted(gpugi_ctx* ctx, const gpugi_nrc* nn, const
             tcAttr = true;
         }
         const uint64_t tiles = (n + 127) / 128;
-        const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->numSMs * tci::kCtas, (tiles + tci::kChains - 1) / tci::kChains);
+        const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->numSMs * tci::kCtas, tiles);
         k<<<(unsigned)grid, 128 * tci::kChains, tci::kSmem, ctx->stream>>>(queries, n, count, nn->wInfT, nn->boxMin,
                                                                            nn->boxInv, out, ctx->errWord, nn->waitNs,
                                                                            nn->stall);
