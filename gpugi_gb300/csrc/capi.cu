@@ -239,7 +239,6 @@ static gpugi_status trace_host(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHi
             const uint64_t mp = std::min(per, m - p0);
             cudaStream_t cs = (p & 1u) ? ctx->compute2 : ctx->stream;
             GPUGI_CUDA_TRY(ctx, cudaStreamWaitEvent(cs, ctx->evIn[p], 0));
-            GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(counters + 4 * p, 0, 4 * sizeof(unsigned long long), cs));
             if ((st = launch_trace_filtered_on(ctx, sc, anyHit, d[0] + p0, d[1] + p0, d[2] + p0, d[3] + p0, d[4] + p0,
                                                d[5] + p0, d[6] + p0, mp, anyHit ? nullptr : dSlot + p0,
                                                anyHit ? nullptr : dT + p0, anyHit ? nullptr : dU + p0,
@@ -491,7 +490,6 @@ static gpugi_status trace_async(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyH
     gpugi_ctx::StreamScratch* ss = nullptr;
     gpugi_status st = stream_scratch(ctx, s, n, &ss);
     if (st) return st;
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(ss->counters, 0, 4 * sizeof(unsigned long long), s));
     st = launch_trace_filtered_on(ctx, sc, anyHit, ox, oy, oz, dx, dy, dz, tmax, n, slot, t, u, v, occluded,
                                   ss->queue, ss->counters, s, ctx->asyncWalkerShare);
     if (st) return st;
@@ -535,7 +533,6 @@ static gpugi_status trace_host_async(gpugi_ctx* ctx, const gpugi_scene* sc, bool
     float* dU = reinterpret_cast<float*>(base + 9 * col);
     float* dV = reinterpret_cast<float*>(base + 10 * col);
     uint8_t* dOcc = reinterpret_cast<uint8_t*>(base + 7 * col);
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(ss->counters, 0, 4 * sizeof(unsigned long long), s));
     st = launch_trace_filtered_on(ctx, sc, anyHit, d[0], d[1], d[2], d[3], d[4], d[5], d[6], n,
                                   anyHit ? nullptr : dSlot, anyHit ? nullptr : dT, anyHit ? nullptr : dU,
                                   anyHit ? nullptr : dV, anyHit ? dOcc : nullptr, ss->queue, ss->counters, s);

@@ -73,8 +73,6 @@ extern "C" gpugi_status gpugi_trace_closest_noalloc(gpugi_ctx* ctx, const gpugi_
     NoAllocScratch s;
     gpugi_status st = resolve_scratch(ctx, s);
     if (st) return st;
-    // The counters keep the previous call's values: clear them on the stream.
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(s.counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
     return launch_trace_filtered_on(ctx, sc, false, ox, oy, oz, dx, dy, dz, tmax, n, slot, t, u, v, nullptr, s.queue,
                                     s.counters);
 }

@@ -4,6 +4,7 @@
 // load and store of a warp is a single coalesced 128-B transaction. The
 // walk itself reads 32-B nodes and 48-B triangle records through the
 // read-only (non-coherent) path with 16-B vector loads.
+#include <algorithm>
 #include <type_traits>
 
 #include "ctx.cuh"
@@ -379,6 +380,41 @@ __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide(
         });
 }
 
+// At most kDirectRays rays per warp of the full grid, on scenes with a wide
+// hierarchy: each ray by a whole warp, straight from the caller's arrays. The
+// prefilter saves one round of such a walk, its launch and the counters' cost
+// more. Measured (us, prefilter and queue / direct; rays aimed at a
+// 4k-triangle object, at a 65k one, and random ones that mostly miss it):
+// 1,000 rays 18.4 / 12.3; 4,865 24.7 / 12.7, 36.3 / 24.7, 30.7 / 19.5; 9,000
+// 26.7 / 19.6, 41.6 / 37.0, 26.7 / 22.6; 20,000 40.5 / 34.8, 61.4 / 63.1, 26.7 /
+// 30.4: the line lies at two rays per warp.
+constexpr uint64_t kDirectRays = 2;
+template <bool ANY_HIT, int TRI>
+__global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide_direct(
+    DevScene s, const float* __restrict__ ox, const float* __restrict__ oy, const float* __restrict__ oz,
+    const float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ dz,
+    const float* __restrict__ tmax, uint32_t n, int32_t* __restrict__ slot, float* __restrict__ t,
+    float* __restrict__ u, float* __restrict__ v, uint8_t* __restrict__ occluded, uint32_t* err) {
+    __shared__ WideShared sh;
+    wide_walks<ANY_HIT, TRI>(
+        sh, s, n, nullptr, err,
+        [&](uint32_t i, float3& o, float3& d, float& len) {
+            o = make_float3(__ldg(ox + i), __ldg(oy + i), __ldg(oz + i));
+            d = make_float3(__ldg(dx + i), __ldg(dy + i), __ldg(dz + i));
+            len = __ldg(tmax + i);
+        },
+        [&](uint32_t i, int32_t hitSlot, float hitT, float hitU, float hitV) {
+            if (ANY_HIT) {
+                occluded[i] = hitSlot >= 0 ? 1 : 0;
+            } else {
+                slot[i] = hitSlot;
+                t[i] = hitT;
+                u[i] = hitU;
+                v[i] = hitV;
+            }
+        });
+}
+
 // Second launch of mode 3 on scenes without a wide hierarchy: 8-lane groups
 // for short queues, one lane per ray for long ones.
 template <bool ANY_HIT, int BOUNDS, int TRI>
@@ -431,13 +467,13 @@ gpugi_status launch_trace_filtered(gpugi_ctx* ctx, const gpugi_scene* sc, bool a
     gpugi_status st = ensure_queue(ctx, n);
     if (st) return st;
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(ctx->scratch);
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
     return launch_trace_filtered_on(ctx, sc, anyHit, ox, oy, oz, dx, dy, dz, tmax, n, slot, t, u, v, occluded,
                                     ctx->queue, counters);
 }
 
 // The same two launches as launch_trace_filtered, on scratch memory the
-// caller provides (queue of n entries, 4 zeroed counters); allocates nothing.
+// caller provides (queue of n entries, 4 counters, which it zeroes on the
+// stream); allocates nothing.
 gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* ox,
                                       const float* oy, const float* oz, const float* dx, const float* dy,
                                       const float* dz, const float* tmax, uint64_t n, int32_t* slot, float* t,
@@ -447,6 +483,23 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
     cudaStream_t cs = stream ? stream : ctx->stream;
     const int ell = (int)sc->dev.boundsKind;  // bounds kind: 0 box, 1 ellipsoid, 2 oriented box
     const bool wt = sc->dev.triangleTest != 0;
+    if (ctx->traceMode == 3 && sc->dev.wide) {
+        auto kd = anyHit ? (wt ? &k_trace_wide_direct<true, 1> : &k_trace_wide_direct<true, 0>)
+                         : (wt ? &k_trace_wide_direct<false, 1> : &k_trace_wide_direct<false, 0>);
+        WalkerLaunch L;
+        gpugi_status st = walker_launch_config(ctx, sc, (const void*)kd, 1ull << 40, 0, L);
+        if (st) return st;
+        if (n <= kDirectRays * 4ull * L.grid) {  // no queue, no counters, one launch
+            const uint64_t spread = n < (uint64_t)ctx->numSMs ? n : (uint64_t)ctx->numSMs;
+            const uint64_t blocks = std::max<uint64_t>((n + 3) / 4, spread);
+            const unsigned grid = (unsigned)std::min<uint64_t>(blocks, L.grid);
+            kd<<<grid, 128, 0, cs>>>(sc->dev, ox, oy, oz, dx, dy, dz, tmax, (uint32_t)n, slot, t, u, v, occluded,
+                                     ctx->errWord);
+            GPUGI_CUDA_TRY(ctx, cudaGetLastError());
+            return GPUGI_OK;
+        }
+    }
+    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), cs));
     // four rays per thread with 16-B accesses when every array allows it
     auto al = [](const void* p) { return p == nullptr || ((uintptr_t)p & 15u) == 0; };
     const bool vec = al(ox) && al(oy) && al(oz) && al(dx) && al(dy) && al(dz) && al(tmax) && al(slot) && al(t) &&

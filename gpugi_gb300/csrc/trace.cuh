@@ -735,7 +735,8 @@ GPUGI_D void leaf_rounds(unsigned todo, const float4 (*ray)[128], const uint32_t
 // ones come from an atomic counter *work, which starts at 0. load(i, o, d,
 // tmax) fills the ray of item i (again when a walk restarts); finish(i, slot,
 // t, u, v) takes its result (any hit: slot >= 0 when occluded). n < 2^32.
-// MULTI: the items belong to several scenes, load returns the item's (a scene
+// work may be null where every warp gets at most kWideSolo items: they are
+// then strided over the warps. MULTI: the items belong to several scenes, load returns the item's (a scene
 // with a wide hierarchy); otherwise every ray walks `scene`.
 template <bool ANY_HIT, int TRI, bool MULTI = false, typename Load, typename Finish>
 GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsigned long long* work, uint32_t* err, Load load,
@@ -1123,6 +1124,10 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
         __syncwarp();
         if (lane == src) active = false;
         if (solo) {
+            if (!work) {
+                next += warps;
+                continue;
+            }
             if (lane == 0) next = warps + atomicAdd(work, 1ull);
             next = __shfl_sync(0xffffffffu, next, 0);
         }

@@ -215,3 +215,25 @@ def test_passes_and_batches(ctx, size, samples):
         assert np.abs(a - z).max() <= 512 * 2.0 ** -24 * max(1.0, float(np.abs(z).max()))
     for s in sets:
         s.close()
+
+
+@pytest.mark.parametrize("n", [1, 151, 153, 607, 609, 9728, 9729])
+def test_direct_and_queued_small_calls(ctx, n):
+    """Both sides of the rule between one launch and prefilter plus queue (two rays per warp of the
+    full grid, 9,728 on 152 SMs), one block per SM and one more; unaligned arrays; a caller's stream."""
+    import torch
+    s = scenes.closed_icosphere(4, seed=2)
+    ds = ctx.build_scene(s["positions"], s["triangles"])
+    rays = special_rays(s["positions"], n, n)
+    want = both_modes(ctx, ds, rays)[1]
+    dev = {k: torch.from_numpy(np.concatenate([v[:1], v])).cuda()[1:] for k, v in rays.items()}  # 4-B aligned
+    out = {k: torch.zeros(n + 1, dtype=torch.int32 if k == "slot" else torch.float32, device="cuda")[1:]
+           for k in ("slot", "t", "u", "v")}
+    occ = torch.zeros(n + 1, dtype=torch.uint8, device="cuda")[1:]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    cuda.trace_closest_device_async(ctx, ds, dev, out, stream.cuda_stream)
+    cuda.trace_any_device_async(ctx, ds, dev, occ, stream.cuda_stream)
+    torch.cuda.synchronize()
+    same(({k: v.cpu().numpy() for k, v in out.items()}, occ.cpu().numpy()), want)
+    ds.close()
