@@ -116,7 +116,8 @@ static uint32_t relayout_nodes(std::vector<float>& nodes, uint32_t numNodes, uin
 }
 
 template <typename T>
-static gpugi_status upload(gpugi_ctx* ctx, gpugi_scene* sc, const T* host, size_t count, const T** dst) {
+static gpugi_status upload(gpugi_ctx* ctx, gpugi_scene* sc, const T* host, size_t count, const T** dst,
+                           bool zero = true) {
     *dst = nullptr;
     if (count == 0) return GPUGI_OK;
     void* p = nullptr;
@@ -125,7 +126,7 @@ static gpugi_status upload(gpugi_ctx* ctx, gpugi_scene* sc, const T* host, size_
     sc->allocations.push_back(p);
     if (host) {
         GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(p, host, count * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
-    } else {
+    } else if (zero) {
         GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(p, 0, count * sizeof(T), ctx->stream));
     }
     *dst = static_cast<const T*>(p);
@@ -236,7 +237,7 @@ extern "C" gpugi_status gpugi_scene_upload(gpugi_ctx* ctx, const float* hierarch
         (st = upload(ctx, sc, reinterpret_cast<const float4*>(materials), 6 * (size_t)numMaterials, &dMat)))
         return cleanup(st);
     const float4* dTris;
-    if ((st = upload<float4>(ctx, sc, nullptr, 3 * (size_t)numSlots, &dTris))) return cleanup(st);
+    if ((st = upload<float4>(ctx, sc, nullptr, 3 * (size_t)numSlots, &dTris, false))) return cleanup(st);
     k_prepare_triangles<<<(numSlots + 255) / 256, 256, 0, ctx->stream>>>(dSlots, numSlots, dPos,
                                                                          const_cast<float4*>(dTris));
     cudaError_t e = cudaGetLastError();
