@@ -40,6 +40,12 @@
 namespace gpugi {
 
 constexpr int kMaxDepth = 64;
+// Resident blocks per SM that the path and light shading kernels are compiled
+// for: bound by latency and instruction fetches, they gain more from warps in
+// flight than the few spilled registers cost (registers as needed / 6 / 7 / 8 /
+// 10 blocks: light-traced room 4.96 / 4.66 / 4.64 / 4.63 / 4.73 ms, thumbnails
+// 2.87 / 2.83 / 2.79 / 2.78 / 2.78, path-traced room 8.89 / 8.90 / 8.85 / 8.83 / 8.94).
+constexpr int kShadeBlocks = 8;
 
 struct PathSoA {
     float *ox, *oy, *oz, *dx, *dy, *dz, *tx, *ty, *tz, *lastP;
@@ -523,7 +529,7 @@ GPUGI_D void pt_shade_lane(const RenderConst& rc, const PathSoA& A, const HitSoA
     L.survive = roulette(rc, depth, thr, L.tp, L.seed) && depth + 1 < rc.maxPathLength;
 }
 
-__global__ void __launch_bounds__(128) k_pt_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q,
+__global__ void __launch_bounds__(128, kShadeBlocks) k_pt_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q,
                                                   int depth) {
     const uint32_t n = rc.cnt->path[depth];
     WARP_LOOP(n, k, valid) {
@@ -624,7 +630,7 @@ GPUGI_D void light_shade_lane(const RenderConst& rc, const PathSoA& A, const Hit
     L.o = L.o + L.d * kRAY_HIT_EPSILON;
 }
 
-__global__ void __launch_bounds__(128) k_light_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q,
+__global__ void __launch_bounds__(128, kShadeBlocks) k_light_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q,
                                                      int depth, bool withCache) {
     const uint32_t n = rc.cnt->path[depth];
     WARP_LOOP(n, k, valid) {
@@ -1938,7 +1944,7 @@ __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_batch_shadow_wid
 
 // One bounce of the phase-0 paths: PT eye paths, LT particles and BPT light
 // paths (the latter append to their job's light cache).
-__global__ void __launch_bounds__(128) k_batch_shade(const RenderConst* __restrict__ jobs, Counters* cnt,
+__global__ void __launch_bounds__(128, kShadeBlocks) k_batch_shade(const RenderConst* __restrict__ jobs, Counters* cnt,
                                                      PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q, int depth) {
     const uint32_t n = cnt->path[depth];
     WARP_LOOP(n, k, valid) {
