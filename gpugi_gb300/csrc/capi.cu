@@ -91,13 +91,6 @@ static gpugi_status ensure_pipeline(gpugi_ctx* ctx) {
     return GPUGI_OK;
 }
 
-// Ray queries on host arrays. Rays go through device staging in chunks of at
-// most 2^22. With trace modes 2-5 a chunk is split into ctx->hostParts parts
-// whose copies in (copyIn stream), traversal (the context stream and a second
-// one, alternating by part) and copies out (copyOut stream) overlap: part p+1
-// uploads while part p is traced, part p downloads while part p+1 is traced,
-// and the traversals of neighbouring parts overlap too. Each part has its own
-// queue range and counters. Returns when every result is in host memory.
 // Device address of page-locked host memory (cudaHostAlloc / cudaHostRegister),
 // or nullptr for any other memory.
 static void* mapped_host(const void* p) {
@@ -107,6 +100,15 @@ static void* mapped_host(const void* p) {
         return nullptr;
     }
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+}
+// Memory that the runtime does not know: pageable host memory.
+static bool plain_host(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
 }
 
 // Copies `count` columns of `width` bytes between host and device. When
@@ -164,6 +166,51 @@ static gpugi_status copy_results_out(gpugi_ctx* ctx, bool anyHit, char* const dR
     return copy_columns(ctx, dst, from, 4, m * 4, cudaMemcpyDeviceToHost, s);
 }
 
+// One traversal that reads the rays and writes the results over the host link,
+// through device addresses of page-locked memory; waits for the results.
+static gpugi_status trace_mapped(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* const d[7], uint64_t n,
+                                 void* const out[4]) {
+    gpugi_status st = anyHit ? launch_trace_any(ctx, sc, d[0], d[1], d[2], d[3], d[4], d[5], d[6], n,
+                                                static_cast<uint8_t*>(out[0]))
+                             : launch_trace_closest(ctx, sc, d[0], d[1], d[2], d[3], d[4], d[5], d[6], n,
+                                                    static_cast<int32_t*>(out[0]), static_cast<float*>(out[1]),
+                                                    static_cast<float*>(out[2]), static_cast<float*>(out[3]));
+    if (st) return st;
+    GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->errHost, ctx->errWord, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    return GPUGI_OK;
+}
+
+// Calls of at most kBounceRays rays in pageable arrays pass through a
+// page-locked block of the context (44 B per ray): the host copies the columns
+// into it and the results out of it, and the kernels work on it over the link. The eleven staged
+// copies cost 5-9 us each however small they are, the host's own copies 3 us
+// per 1,000 rays (icosphere of 65k triangles, closest hit, staged / through the
+// block: 1 ray 81 / 40 us, 1,000 75 / 54, 8,192 93 / 82, 16,384 155 / 128; at
+// twice that the two meet). Page-locked arrays are copied faster than that
+// (4,000 rays 55 / 60 us, 16,384 86 / 127).
+constexpr uint64_t kBounceRays = 16384;
+static bool ensure_bounce(gpugi_ctx* ctx) {
+    if (ctx->bounceDev) return true;
+    void* dev = nullptr;
+    if (!ctx->bounce && cudaMallocHost(&ctx->bounce, kBounceRays * 44) != cudaSuccess) ctx->bounce = nullptr;
+    if (ctx->bounce && cudaHostGetDevicePointer(&dev, ctx->bounce, 0) == cudaSuccess) ctx->bounceDev = dev;
+    if (!ctx->bounceDev) cudaGetLastError();  // the staged copies serve as well
+    return ctx->bounceDev != nullptr;
+}
+
+// Ray queries on host arrays. Rays go through device staging in chunks of at
+// most 2^22. With trace modes 2-5 a chunk of page-locked arrays is split into
+// ctx->hostParts parts whose copies in (copyIn stream), traversal (the context
+// stream and a second one, alternating by part) and copies out (copyOut
+// stream) overlap: part p+1 uploads while part p is traced, part p downloads
+// while part p+1 is traced, and the traversals of neighbouring parts overlap
+// too. Each part has its own queue range and counters. Copies of pageable
+// memory keep the host waiting and overlap with next to nothing, so such
+// arrays stay in one part (aimed rays at the icosphere of 65k triangles, one /
+// two parts: 300k rays 436 / 528 us, 2^20 1.26 / 1.32 ms, 2^22 4.46 / 4.39 ms;
+// page-locked 2^20 1.16 / 1.09 ms, 2^22 4.28 / 3.87 ms). Returns when every
+// result is in host memory.
 static gpugi_status trace_host(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* const src[7],
                                uint64_t n, int32_t* slot, float* t, float* u, float* v, uint8_t* occ) {
     // Page-locked arrays: the kernels read the rays and write the results
@@ -178,18 +225,28 @@ static gpugi_status trace_host(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHi
             void* outs[4] = {slot, t, u, v};
             for (int k = 0; k < 4 && ok; ++k) ok = (dout[k] = mapped_host(outs[k])) != nullptr;
         }
-        if (ok) {
-            gpugi_status st = anyHit ? launch_trace_any(ctx, sc, dsrc[0], dsrc[1], dsrc[2], dsrc[3], dsrc[4], dsrc[5],
-                                                        dsrc[6], n, static_cast<uint8_t*>(dout[0]))
-                                     : launch_trace_closest(ctx, sc, dsrc[0], dsrc[1], dsrc[2], dsrc[3], dsrc[4],
-                                                            dsrc[5], dsrc[6], n, static_cast<int32_t*>(dout[0]),
-                                                            static_cast<float*>(dout[1]), static_cast<float*>(dout[2]),
-                                                            static_cast<float*>(dout[3]));
-            if (st) return st;
-            GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->errHost, ctx->errWord, 4, cudaMemcpyDeviceToHost, ctx->stream));
-            GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-            return GPUGI_OK;
+        if (ok) return trace_mapped(ctx, sc, anyHit, dsrc, n, dout);
+    }
+    void* const outs[4] = {anyHit ? static_cast<void*>(occ) : slot, t, u, v};
+    const int numOut = anyHit ? 1 : 4;
+    // only plain memory: the host itself reads and writes the arrays there
+    bool plain = n <= kBounceRays;
+    for (int k = 0; k < 7 && plain; ++k) plain = plain_host(src[k]);
+    for (int k = 0; k < numOut && plain; ++k) plain = plain_host(outs[k]);
+    if (plain && ensure_bounce(ctx)) {
+        char* host = static_cast<char*>(ctx->bounce);
+        char* dev = static_cast<char*>(ctx->bounceDev);
+        const size_t col = kBounceRays * 4;
+        const float* dsrc[7];
+        void* dout[4];
+        for (int k = 0; k < 7; ++k) {
+            memcpy(host + k * col, src[k], n * 4);
+            dsrc[k] = reinterpret_cast<const float*>(dev + k * col);
         }
+        for (int k = 0; k < 4; ++k) dout[k] = dev + (7 + k) * col;
+        if (gpugi_status st = trace_mapped(ctx, sc, anyHit, dsrc, n, dout)) return st;
+        for (int k = 0; k < numOut; ++k) memcpy(outs[k], host + (7 + k) * col, anyHit ? n : n * 4);
+        return GPUGI_OK;
     }
     const uint64_t chunk = n < (1ull << 22) ? n : (1ull << 22);
     const size_t col = align256(chunk * 4);
@@ -205,7 +262,7 @@ static gpugi_status trace_host(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHi
     uint8_t* dOcc = reinterpret_cast<uint8_t*>(base + 7 * col);
     char* const dRes[4] = {base + 7 * col, base + 8 * col, base + 9 * col, base + 10 * col};
     const uint32_t parts = std::min<uint32_t>(std::max<uint32_t>(ctx->hostParts, 1u), 8u);
-    const bool pipe = ctx->traceMode >= 2 && parts > 1 && chunk >= (1ull << 16);
+    const bool pipe = ctx->traceMode >= 2 && parts > 1 && chunk >= (1ull << 16) && mapped_host(src[0]) && mapped_host(outs[0]);
     if (pipe) {
         if ((st = ensure_pipeline(ctx)) || (st = ensure_queue(ctx, chunk))) return st;
     }
@@ -314,6 +371,7 @@ void gpugi_destroy(gpugi_ctx* ctx) {
     if (ctx->stageDev) cudaFree(ctx->stageDev);
     if (ctx->errWord) cudaFree(ctx->errWord);
     if (ctx->errHost) cudaFreeHost(ctx->errHost);
+    if (ctx->bounce) cudaFreeHost(ctx->bounce);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->queue) cudaFree(ctx->queue);
     for (auto& ss : ctx->streamScratch) {

@@ -21,6 +21,9 @@ struct gpugi_ctx {
     // staging for the host-pointer entry points (grown on demand)
     void* stageDev = nullptr;
     size_t stageDevBytes = 0;
+    // page-locked block of small host-array queries, made at the first one
+    void* bounce = nullptr;
+    void* bounceDev = nullptr;  // its device address
     // trace tuning
     uint32_t traceMode = 3;  // 0 thread per ray, 1 persistent lane refill, 2 root prefilter + 1, 3 + wide walk or 8-lane groups, 4/5 + 4/16-lane groups
     uint32_t traceBlock = 128;

@@ -516,3 +516,30 @@ def test_stream_ordered_queries_on_many_streams(cuda_ctx, icosphere_65536):
             _compare_closest({k: v.cpu().numpy() for k, v in outs[i].items()}, cuda.trace_closest(cuda_ctx, ds, host[i]))
     assert cuda_ctx.device_error_bits() == 0
     ds.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 9729, 16384, 16385, 65537])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_host_arrays_of_each_size(cuda_ctx, icosphere_65536, n, shift):
+    """Pageable host arrays on both sides of the page-locked block's size and of the split into
+    parts, also one float off a 16-B boundary: the device arrays' results, bit for bit."""
+    import torch
+    sc = icosphere_65536
+    b = bvh.build_bvh(sc["positions"], sc["triangles"], method="sweep")
+    ds = cuda_ctx.upload_scene(b, sc["positions"])
+    rays = {k: np.concatenate([np.zeros(shift, np.float32), v])[shift:] for k, v in
+            scenes.aimed_rays(n, sc["positions"], seed=n, spread=2.5).items()}
+    dev = {k: torch.from_numpy(v.copy()).cuda() for k, v in rays.items()}
+    want = {k: torch.empty(n, dtype=torch.int32 if k == "slot" else torch.float32, device="cuda")
+            for k in ("slot", "t", "u", "v")}
+    occ = torch.empty(n, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    cuda.trace_closest_device(cuda_ctx, ds, dev, want)
+    cuda.trace_any_device(cuda_ctx, ds, dev, occ)
+    got = cuda.trace_closest(cuda_ctx, ds, rays)
+    got_occ = cuda.trace_any(cuda_ctx, ds, rays)
+    torch.cuda.synchronize()
+    for k in want:
+        np.testing.assert_array_equal(got[k].view(np.uint32), want[k].cpu().numpy().view(np.uint32), err_msg=k)
+    np.testing.assert_array_equal(got_occ, occ.cpu().numpy())
+    ds.close()
