@@ -42,7 +42,7 @@ FALLBACK_HBM_GBS = 6800.0
 # Kernels of one step per trace mode (the roofline is taken over the whole step).
 KERNELS = {0: "k_trace_closest<AABB>", 1: "k_trace_persistent<closest, AABB>",
            2: "k_trace_root_filter<closest, AABB> + k_trace_queue<closest, AABB>",
-           3: "k_trace_root_filter<closest, AABB> + k_trace_group<closest, AABB, 8>",
+           3: "k_trace_root_filter<closest, AABB> + k_trace_wide<closest>",
            4: "k_trace_root_filter<closest, AABB> + k_trace_group<closest, AABB, 4>",
            5: "k_trace_root_filter<closest, AABB> + k_trace_group<closest, AABB, 16>"}
 
@@ -1227,7 +1227,7 @@ def main():
                     help="streams the end-to-end host-buffer steps alternate over")
     ap.add_argument("--trace-mode", type=int, default=3,
                     help="0: thread per ray, 1: persistent lane refill, 2: root prefilter + persistent, "
-                         "3/4/5: root prefilter + 8/4/16-lane group walker")
+                         "3: root prefilter + wide walker, 4/5: root prefilter + 4/16-lane group walker")
     ap.add_argument("--batch-seed", type=int, default=1)
     ap.add_argument("--host-parts", type=int, default=2,
                     help="parts of a host-pointer query whose copies and traversal overlap")

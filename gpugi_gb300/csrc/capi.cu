@@ -433,7 +433,7 @@ gpugi_status gpugi_set_trace_config(gpugi_ctx* ctx, uint32_t mode, uint32_t bloc
     if (mode > 5)
         return fail(ctx, GPUGI_ERROR_INVALID_ARGUMENT,
                     "mode must be 0 (thread per ray), 1 (persistent), 2 (root prefilter + persistent) or "
-                    "3/4/5 (root prefilter + 8/4/16-lane group walker)");
+                    "3 (root prefilter + wide or 8-lane walk) or 4/5 (root prefilter + 4/16-lane group walker)");
     if (blockSize == 0 || blockSize > 256 || blockSize % 32 != 0)
         return fail(ctx, GPUGI_ERROR_INVALID_ARGUMENT, "blockSize must be a multiple of 32 in [32, 256]");
     ctx->traceMode = mode;

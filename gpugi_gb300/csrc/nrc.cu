@@ -488,8 +488,12 @@ __global__ void k_nrc_encode(const float* __restrict__ queries, uint64_t n, floa
 }
 
 // ------------------------------------------------ tcgen05 training kernel
-// One CTA per SM runs 128-sample tiles: thread t owns sample t of a tile
-// (TMEM lane t). Per tile, ten MMA phases, each issued by thread 0 and
+// One CTA of 256 threads per SM runs 128-sample tiles: threads t and t + 128
+// share sample t of a tile (TMEM lane t), each taking half of its features in
+// the encoding and of the columns between the phases. Bound by the latency of
+// the ten phases, which wait for one another, at 8 warps per SM (the operands
+// of all layers fill the shared memory); one thread per sample took 45.6 us
+// for 65,536 samples, two take 37. Per tile, ten MMA phases, each issued by thread 0 and
 // completed through one mbarrier: forward layers 0-4 (D = X_l W_l), backward
 // layers 4-1 (D = dY_l W_l^T), then the weight gradients of the tile,
 // accumulated in TMEM across all tiles of the CTA. Between phases the
@@ -941,7 +945,7 @@ __global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc
 // groups of it in parallel, then the four group sums in order; ADAM: the
 // optimiser's step follows in the same launch. Block 0 also sums the CTAs'
 // losses. Bound by the latency of the row reads (10.6 MB from L2): 16 of them
-// in flight per thread and the step fused, 5.1 us instead of 7.0 + 5.1 us.
+// in flight per thread and the step fused, 7.3 us instead of 7.0 + 5.1 us.
 template <bool ADAM>
 __global__ void __launch_bounds__(256) k_nrc_sum_partials(const float* __restrict__ partials,
                                                           const float* __restrict__ lossPart, int rows,

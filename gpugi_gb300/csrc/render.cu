@@ -31,8 +31,8 @@
 #include "shade.cuh"
 #include "trace.cuh"
 
-// The passes' walkers walk a queue with 8-lane groups while it holds fewer
-// rays than this many times the resident lanes, and a ray per lane otherwise.
+// On scenes without a wide hierarchy the passes' walkers walk a queue with
+// 8-lane groups while it holds fewer rays than this many times the resident lanes, and a ray per lane otherwise.
 #ifndef GPUGI_GROUP_BELOW_LANES
 #define GPUGI_GROUP_BELOW_LANES 2u
 #endif
@@ -326,8 +326,9 @@ __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_shadow_wide(Rend
         });
 }
 
-// Launch shapes and launches of the walkers for a scene: group walks when the
-// context's trace mode is 3 or 4, else lane walks with staged top nodes.
+// Launch shapes and launches of the walkers for a scene: the wide walk in trace
+// mode 3 where the scene has the wide hierarchy; else, in modes 3-5, group walks
+// of short queues and lane walks of long ones; lane walks in modes 0-2.
 struct Walkers {
     int bounds = 0;  // node kind: 0 box, 1 ellipsoid, 2 oriented box
     bool wide = false;  // walks on the wide hierarchy

@@ -591,7 +591,7 @@ GPUGI_D void group_walks_multi(uint64_t n, unsigned long long* work, uint32_t* e
 // Walks over the four-wide copy of an axis-aligned-box hierarchy (wide.cu):
 // depth first with a stack of {reference, entry distance}, children in
 // preorder, so leaves are met in exactly the order of the escape walk. The
-// results are trace_ray's bit for bit although every second level is left
+// results are trace_ray's bit for bit although most inner levels are left
 // out and four boxes are tested per fetch:
 //  * The escape walk tests a leaf's triangles iff the leaf's box and all its
 //    ancestors' boxes are hit with firstHit <= rayLength when they are met.
@@ -621,13 +621,13 @@ GPUGI_D void group_walks_multi(uint64_t n, unsigned long long* work, uint32_t* e
 // groups on 8-wide nodes issued 2.3x the instructions); leaves go to eight
 // lanes each, four leaves at a time, because a lane that loops over a block's
 // triangles waits for memory once per triangle (1.05 to 0.87 ms for 3M
-// any-hit rays in the 528k-triangle terrain). Quantised 96-B nodes halved
+// any-hit rays in the 528k-triangle terrain, then). Quantised 96-B nodes halved
 // the L1 load but cost more issue slots than they freed (0.99 ms); prefetches
 // of waiting children cost 2-8 %.
 // Measured against the binary walkers: 3M any-hit rays in the terrain
-// 2.19 to 0.85 ms, path tracing the room at 512^2 x 16 samples 15.98 to
-// 9.3 ms, light tracing 9.16 to 5.3 ms, 1,000 rays (a warp each) 43 to 18 us, a
-// 320 x 180 frame 1.03 to 0.63 ms (0.92 with eight lanes per ray at the end).
+// 2.18 to 0.80 ms, path tracing the room at 512^2 x 16 samples 15.7 to 8.8 ms,
+// light tracing 9.0 to 4.6 ms, 1,000 rays (a warp each) 42.3 to 12.1 us, a
+// 320 x 180 frame 1.03 to 0.60 ms (0.92 with eight lanes per ray at the end).
 GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
 
 // Lanes of a warp step through nodes together until kWideLeaves leaves wait or
