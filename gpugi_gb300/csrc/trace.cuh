@@ -641,9 +641,11 @@ GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfini
 // 137 / 129 / 120 / 118 / 123 for 66k rays in the icosphere). Queues of at most
 // kWideSolo rays per warp are walked that way from the start (1 / 4 / 8 / 16 /
 // 32: 664 / 655 / 623 / 616 / 617 us for the frame; 119 / 127 us at 8 / 16 for
-// the icosphere's 66k).
+// the icosphere's 66k) or, since any-hit walks end early, kWideSoloAny
+// (30,000 rays at 8 / 5: 36.3 / 29.5 us in a room of 3k triangles, 40.2 / 33.6 in
+// one of 20k; 20,000 at 5 / 4: 34.8 / 38.4 in a terrain of 100k).
 constexpr int kWideLeaves = 8, kWideNodes = 8, kWideRefill = 12, kWideWarpAt = 5;
-constexpr uint32_t kWideSolo = 8;
+constexpr uint32_t kWideSolo = 8, kWideSoloAny = 5;
 // Resident blocks per SM that the wide walkers are compiled for (64
 // registers; 7 / 8 / 9 blocks: 9.94 / 9.60 / 9.63 ms for the path-traced room).
 #ifndef GPUGI_WIDE_MIN_BLOCKS
@@ -834,7 +836,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
     const uint64_t first = (uint64_t)warps * C;
     bool more = n > first;
     const uint64_t warp = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const bool solo = n <= (uint64_t)warps * kWideSolo;
+    const bool solo = n <= (uint64_t)warps * (ANY_HIT ? kWideSoloAny : kWideSolo);
     if (!solo) {
         const uint64_t i = warp * C + lane;
         if (lane < C && i < n) begin((uint32_t)i);
