@@ -318,18 +318,20 @@ __global__ void __launch_bounds__(128) k_trace_queue(
     }
 }
 
-// Group walker (modes 4 and 5), second launch after the root prefilter: G
-// lanes walk each queued ray together (group_step), which shortens the
-// dependent fetch chain of the longest walks.
+// Group walker, a launch after the root prefilter: G lanes walk each queued
+// ray together (group_step), which shortens the dependent fetch chain of the
+// longest walks. Queues of `limit` rays and more are left to k_trace_lanes.
 template <bool ANY_HIT, int BOUNDS, int G, int TRI>
 __global__ void __launch_bounds__(128, GPUGI_GROUP_MIN_BLOCKS) k_trace_group(
     DevScene s, const float* __restrict__ ox, const float* __restrict__ oy, const float* __restrict__ oz,
     const float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ dz,
     const float* __restrict__ tmax, int32_t* __restrict__ slot, float* __restrict__ t, float* __restrict__ u,
     float* __restrict__ v, uint8_t* __restrict__ occluded, const uint32_t* __restrict__ queue,
-    unsigned long long* counters, uint32_t* err) {
+    unsigned long long* counters, uint32_t* err, uint64_t limit) {
+    const uint64_t n = counters[1];
+    if (n >= limit) return;
     group_walks<ANY_HIT, BOUNDS, G, TRI>(
-        s, counters[1], counters + 2, err,
+        s, n, counters + 2, err,
         [&](uint64_t i, float3& o, float3& d, float& len) {
             const uint32_t ray = __ldg(queue + i);
             o = make_float3(__ldg(ox + ray), __ldg(oy + ray), __ldg(oz + ray));
@@ -415,40 +417,41 @@ __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide_direc
         });
 }
 
-// Second launch of mode 3 on scenes without a wide hierarchy: 8-lane groups
-// for short queues, one lane per ray for long ones.
+// Mode 3 on scenes without a wide hierarchy, queues of `from` rays and more
+// (shorter ones are k_trace_group's, which is launched with it): one lane per
+// ray. Two kernels because the walks want different numbers of blocks per SM:
+// in one kernel compiled for 8, groups took 3-5 % longer than at their 10, and
+// at 9 or 10 lanes lost as much; the launch that finds nothing to do costs
+// less, and calls that cannot fill the queue that far skip it.
 template <bool ANY_HIT, int BOUNDS, int TRI>
-__global__ void __launch_bounds__(128, 8) k_trace_binary(
+__global__ void __launch_bounds__(128, 8) k_trace_lanes(
     DevScene s, const float* __restrict__ ox, const float* __restrict__ oy, const float* __restrict__ oz,
     const float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ dz,
     const float* __restrict__ tmax, int32_t* __restrict__ slot, float* __restrict__ t, float* __restrict__ u,
     float* __restrict__ v, uint8_t* __restrict__ occluded, const uint32_t* __restrict__ queue,
-    unsigned long long* counters, uint32_t* err) {
+    unsigned long long* counters, uint32_t* err, uint64_t from) {
     __shared__ LaneShared sh;
     const uint64_t n = counters[1];
-    auto load = [&](uint64_t i, float3& o, float3& d, float& len) {
-        const uint32_t ray = __ldg(queue + i);
-        o = make_float3(__ldg(ox + ray), __ldg(oy + ray), __ldg(oz + ray));
-        d = make_float3(__ldg(dx + ray), __ldg(dy + ray), __ldg(dz + ray));
-        len = __ldg(tmax + ray);
-    };
-    auto finish = [&](uint64_t i, int32_t hitSlot, float hitT, float hitU, float hitV) {
-        const uint32_t ray = __ldg(queue + i);
-        if (ANY_HIT) {
-            occluded[ray] = hitSlot >= 0 ? 1 : 0;
-        } else {
-            slot[ray] = hitSlot;
-            t[ray] = hitT;
-            u[ray] = hitU;
-            v[ray] = hitV;
-        }
-    };
-    if (n < (uint64_t)gridDim.x * GPUGI_LANE_FROM)
-        group_walks<ANY_HIT, BOUNDS, 8, TRI>(s, n, counters + 2, err, load, [&](uint64_t i, const GroupWalk& g) {
-            finish(i, g.slot, g.len, g.u, g.v);
+    if (n < from) return;
+    lane_walks<ANY_HIT, BOUNDS, TRI>(
+        sh, s, n, counters + 2, err,
+        [&](uint64_t i, float3& o, float3& d, float& len) {
+            const uint32_t ray = __ldg(queue + i);
+            o = make_float3(__ldg(ox + ray), __ldg(oy + ray), __ldg(oz + ray));
+            d = make_float3(__ldg(dx + ray), __ldg(dy + ray), __ldg(dz + ray));
+            len = __ldg(tmax + ray);
+        },
+        [&](uint64_t i, int32_t hitSlot, float hitT, float hitU, float hitV) {
+            const uint32_t ray = __ldg(queue + i);
+            if (ANY_HIT) {
+                occluded[ray] = hitSlot >= 0 ? 1 : 0;
+            } else {
+                slot[ray] = hitSlot;
+                t[ray] = hitT;
+                u[ray] = hitU;
+                v[ray] = hitV;
+            }
         });
-    else
-        lane_walks<ANY_HIT, BOUNDS, TRI>(sh, s, n, counters + 2, err, load, finish);
 }
 
 // walkerShare percent of a persistent walker grid (at least one block).
@@ -544,9 +547,25 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
         return GPUGI_OK;
     }
     if (ctx->traceMode >= 3) {
+        uint64_t limit = ~0ull;  // queue length from which lanes walk alone
+        WalkerLaunch L;
+        if (ctx->traceMode == 3) {
+            auto kl = pick_variant(anyHit, ell, wt, [](auto A, auto B, auto T) {
+                return &k_trace_lanes<decltype(A)::value, decltype(B)::value, decltype(T)::value>;
+            });
+            gpugi_status st = walker_launch_config(ctx, sc, (const void*)kl, 1ull << 40, 0, L);
+            if (st) return st;
+            L.grid = share_of_grid(L.grid, walkerShare);
+            limit = (uint64_t)L.grid * GPUGI_LANE_FROM;
+            if (n >= limit) {
+                kl<<<L.grid, 128, 0, cs>>>(sc->dev, ox, oy, oz, dx, dy, dz, tmax, slot, t, u, v, occluded, queue,
+                                           counters, ctx->errWord, limit);
+                GPUGI_CUDA_TRY(ctx, cudaGetLastError());
+            }
+        }
         auto kg = ctx->traceMode == 3
                       ? pick_variant(anyHit, ell, wt, [](auto A, auto B, auto T) {
-                            return &k_trace_binary<decltype(A)::value, decltype(B)::value, decltype(T)::value>;
+                            return &k_trace_group<decltype(A)::value, decltype(B)::value, 8, decltype(T)::value>;
                         })
                   : ctx->traceMode == 4
                       ? pick_variant(anyHit, ell, wt, [](auto A, auto B, auto T) {
@@ -555,12 +574,11 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
                       : pick_variant(anyHit, ell, wt, [](auto A, auto B, auto T) {
                             return &k_trace_group<decltype(A)::value, decltype(B)::value, 16, decltype(T)::value>;
                         });
-        WalkerLaunch L;
         gpugi_status st = walker_launch_config(ctx, sc, (const void*)kg, 1ull << 40, 0, L);
         if (st) return st;
         L.grid = share_of_grid(L.grid, walkerShare);
         kg<<<L.grid, 128, 0, cs>>>(sc->dev, ox, oy, oz, dx, dy, dz, tmax, slot, t, u, v, occluded, queue,
-                                           counters, ctx->errWord);
+                                   counters, ctx->errWord, limit);
         GPUGI_CUDA_TRY(ctx, cudaGetLastError());
         return GPUGI_OK;
     }

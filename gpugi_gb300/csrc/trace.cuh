@@ -1150,13 +1150,15 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
 // ray for windows of which a third is visited. Measured on fitted ellipsoids,
 // 100k instanced triangles, rays from inside (us, 8-lane groups / this):
 // 20,000 rays 143 / 158, 40,000 181 / 199, 60,000 209 / 216, 100,000 281 / 240,
-// 500,000 935 / 458, 2,000,000 3,451 / 1,349. So queues of fewer rays than
-// 56 per block of the full grid (68,000 on 152 SMs) stay with the groups.
+// 500,000 935 / 458, 2,000,000 3,451 / 1,349; a room of 40k triangles 50,000
+// rays 638 / 641, 70,000 737 / 712; an icosphere of 20k 168 / 171, 212 / 184. So
+// queues of fewer rays than 48 per block of the full grid (58,000 on 152 SMs)
+// stay with the groups.
 // Nodes per loop 1 / 2 / 4 / 8: 496 / 489 / 458 / 473 us at 500,000; waiting
 // leaves 2 / 4 / 8: 462 / 458 / 476; handed over at 2 / 3 / 4 rays: 509 / 471
 // / 458.
 #ifndef GPUGI_LANE_FROM
-#define GPUGI_LANE_FROM 56u
+#define GPUGI_LANE_FROM 48u
 #endif
 constexpr int kLaneSteps = 4, kLaneLeaves = 4, kLaneNodes = 8, kLaneRefill = 8, kLaneGroupAt = 4;
 struct LaneShared {
