@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(256, 1) k_nrc_train_tc(const float* __restrict
 }
 
 // ----------------------------------------------- tcgen05 inference kernel
-// tci::kChains warpgroups per CTA, each running its own chain of 128-query
+// CHAINS warpgroups per CTA, each running its own chain of 128-query
 // tiles: thread t of a warpgroup owns query t of the tile (TMEM lane t), one
 // thread per warpgroup issues the five layers' MMAs (D = X W_l) into the
 // warpgroup's 64 TMEM columns and its mbarrier tracks them; between layers
@@ -793,8 +793,12 @@ constexpr uint32_t kWBytes = tcl::kWBytes;
 // chains per CTA x CTAs per SM, a lookup of 921,600 queries through the public call: 2 x 3 106.6 us,
 // 3 x 2 104.7, 1 x 4 111.0, 2 x 4 115.0, 4 x 2 102.7 (109.4 before, 2 x 3 without the early fetch)
 constexpr uint32_t kChains = 4, kCtas = 2;
-constexpr uint32_t kCols = 64 * kChains;  // a power of two
-constexpr uint32_t kSmem = kWBytes + kChains * kXBytes + 1024;
+// At most kFewPerSM tiles per SM, where most chains would have none: smaller CTAs, which start sooner
+// (the kernel, 4 x 2 / 2 x 3: 8,000 queries 9.8 / 8.2 us, 36,822 12.0 / 10.5; 48,000 11.2 / 12.8,
+// 75,000 12.3 / 13.8; one chain 9.2 and 12.8: its 128 threads stage the weights slowly)
+constexpr uint32_t kFewChains = 2, kFewCtas = 3, kFewPerSM = 2;
+constexpr uint32_t cols(uint32_t chains) { return 64 * chains; }  // a power of two
+constexpr uint32_t smem(uint32_t chains) { return kWBytes + chains * kXBytes + 1024; }
 }  // namespace tci
 
 // A barrier of the warpgroup's 128 threads that also ORs a flag over them.
@@ -807,8 +811,8 @@ GPUGI_D bool wg_any(int wg, bool v) {
     return r != 0;
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc(const float* __restrict__ queries, uint64_t n,
+template <bool VEC, uint32_t CHAINS, uint32_t CTAS>
+__global__ void __launch_bounds__(128 * CHAINS, CTAS) k_nrc_infer_tc(const float* __restrict__ queries, uint64_t n,
                                                       const uint32_t* __restrict__ count,
                                                       const __half* __restrict__ wInfT, float3 boxMin, float3 boxInv,
                                                       float* __restrict__ out, uint32_t* errWord, uint64_t waitNs,
@@ -818,7 +822,7 @@ __global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc
     if (count) n = min(n, (uint64_t)*count);
     extern __shared__ uint8_t smemRaw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t bars[tci::kChains];
+    __shared__ uint64_t bars[CHAINS];
     __shared__ uint32_t tmemBase;
     const int t = threadIdx.x, wg = t >> 7, lt = t & 127, warp = t >> 5;
     for (int l = 0; l < kLayers; ++l) {
@@ -830,9 +834,9 @@ __global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc
         }
     }
     if (t == 0) {
-        for (uint32_t k = 0; k < tci::kChains; ++k) bar_init(&bars[k], 1);
+        for (uint32_t k = 0; k < CHAINS; ++k) bar_init(&bars[k], 1);
     }
-    if (warp == 0) tmem_alloc(&tmemBase, tci::kCols);
+    if (warp == 0) tmem_alloc(&tmemBase, tci::cols(CHAINS));
     fence_smem();
     fence_before();
     __syncthreads();
@@ -860,7 +864,7 @@ __global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc
                 p[k] = row < n ? make_float4(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]) : make_float4(0, 0, 0, 0);
         }
     };
-    const uint64_t stride = tci::kChains * (uint64_t)gridDim.x;
+    const uint64_t stride = CHAINS * (uint64_t)gridDim.x;
     // few tiles: one chain of each CTA before the second of any
     uint64_t tile = (uint64_t)wg * gridDim.x + blockIdx.x;
     fetch(tile);
@@ -937,7 +941,7 @@ __global__ void __launch_bounds__(128 * tci::kChains, tci::kCtas) k_nrc_infer_tc
     fence_before();
     __syncthreads();
     fence_after();
-    if (warp == 0) tmem_free(tmemBase, tci::kCols);
+    if (warp == 0) tmem_free(tmemBase, tci::cols(CHAINS));
 }
 
 // grad[i] = sum over the CTAs' partial sums, in a fixed order
@@ -1011,20 +1015,26 @@ gpugi_status gpugi::nrc_infer_counted(gpugi_ctx* ctx, const gpugi_nrc* nn, const
                                       const uint32_t* count, float* out) {
     if (n == 0) return GPUGI_OK;
     if (nn->kernels == GPUGI_NRC_KERNELS_TCGEN05) {
-        auto k = ((uintptr_t)queries & 15u) == 0 ? &k_nrc_infer_tc<true> : &k_nrc_infer_tc<false>;
+        const uint64_t tiles = (n + 127) / 128;
+        const bool vec = ((uintptr_t)queries & 15u) == 0, few = tiles <= (uint64_t)ctx->numSMs * tci::kFewPerSM;
+        using namespace tci;
+        auto k = few ? (vec ? &k_nrc_infer_tc<true, kFewChains, kFewCtas> : &k_nrc_infer_tc<false, kFewChains, kFewCtas>)
+                     : (vec ? &k_nrc_infer_tc<true, kChains, kCtas> : &k_nrc_infer_tc<false, kChains, kCtas>);
         static bool tcAttr = false;
         if (!tcAttr) {
-            GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(k_nrc_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)tci::kSmem));
-            GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(k_nrc_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)tci::kSmem));
+            for (auto f : {&k_nrc_infer_tc<true, kChains, kCtas>, &k_nrc_infer_tc<false, kChains, kCtas>})
+                GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)smem(kChains)));
+            for (auto f : {&k_nrc_infer_tc<true, kFewChains, kFewCtas>, &k_nrc_infer_tc<false, kFewChains, kFewCtas>})
+                GPUGI_CUDA_TRY(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)smem(kFewChains)));
             tcAttr = true;
         }
-        const uint64_t tiles = (n + 127) / 128;
-        const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->numSMs * tci::kCtas, tiles);
-        k<<<(unsigned)grid, 128 * tci::kChains, tci::kSmem, ctx->stream>>>(queries, n, count, nn->wInfT, nn->boxMin,
-                                                                           nn->boxInv, out, ctx->errWord, nn->waitNs,
-                                                                           nn->stall);
+        const uint32_t chains = few ? kFewChains : kChains;
+        const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->numSMs * (few ? kFewCtas : kCtas), tiles);
+        k<<<(unsigned)grid, 128 * chains, smem(chains), ctx->stream>>>(queries, n, count, nn->wInfT, nn->boxMin,
+                                                                       nn->boxInv, out, ctx->errWord, nn->waitNs,
+                                                                       nn->stall);
         GPUGI_CUDA_TRY(ctx, cudaGetLastError());
         return GPUGI_OK;
     }

@@ -194,12 +194,12 @@ def test_training_learns_a_smooth_field(cuda_ctx):
     c.close()
 
 
-@pytest.mark.parametrize("n", [1, 127, 129, 512, 513, 155648, 155649, 160001])
+@pytest.mark.parametrize("n", [1, 127, 129, 512, 513, 38912, 38913, 155648, 155649, 160001])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_inference_sizes_and_alignment(n, shift):
     """The tcgen05 lookups against the mma.sync ones: part tiles, part CTAs, one tile per chain of the
-    full grid (8 x 152 tiles) and one more, records on 16-B and on 4-B boundaries. The same fp16
-    weights, encodings and activations, f32 sums in another order: a sum of 64 terms differs by at
+    full grid (8 x 152 tiles) and one more, as many tiles as the smaller CTAs take (2 x 152) and one
+    more, records on 16-B and on 4-B boundaries. The same fp16 weights, encodings and activations, f32 sums in another order: a sum of 64 terms differs by at
     most 64 * 2^-24 of its absolute terms, which can move an activation by one fp16 step (2^-10
     relative) in each of the four hidden layers."""
     import torch
