@@ -626,8 +626,8 @@ GPUGI_D void group_walks_multi(uint64_t n, unsigned long long* work, uint32_t* e
 // of waiting children cost 2-8 %.
 // Measured against the binary walkers: 3M any-hit rays in the terrain
 // 2.18 to 0.80 ms, path tracing the room at 512^2 x 16 samples 15.7 to 8.8 ms,
-// light tracing 9.0 to 4.6 ms, 1,000 rays (a warp each) 42.3 to 12.1 us, a
-// 320 x 180 frame 1.03 to 0.60 ms (0.92 with eight lanes per ray at the end).
+// light tracing 9.0 to 4.6 ms, 1,000 rays (a warp each) 43.7 to 12.3 us, a
+// 320 x 180 frame 1.03 to 0.62 ms (0.92 with eight lanes per ray at the end).
 GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
 
 // Lanes of a warp step through nodes together until kWideLeaves leaves wait or
@@ -643,7 +643,8 @@ GPUGI_D bool finite3(float3 v) { return isfinite(v.x) && isfinite(v.y) && isfini
 // 32: 664 / 655 / 623 / 616 / 617 us for the frame; 119 / 127 us at 8 / 16 for
 // the icosphere's 66k) or, since any-hit walks end early, kWideSoloAny
 // (30,000 rays at 8 / 5: 36.3 / 29.5 us in a room of 3k triangles, 40.2 / 33.6 in
-// one of 20k; 20,000 at 5 / 4: 34.8 / 38.4 in a terrain of 100k).
+// one of 20k, the frame 608 / 615; 20,000 at 5 / 4: 34.8 / 38.4 in a terrain of
+// 100k).
 constexpr int kWideLeaves = 8, kWideNodes = 8, kWideRefill = 12, kWideWarpAt = 5;
 constexpr uint32_t kWideSolo = 8, kWideSoloAny = 5;
 // Resident blocks per SM that the wide walkers are compiled for (64
