@@ -1000,9 +1000,13 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
             ++wsp;
             __syncwarp();
         }
-        // `leaves` leading leaves, lane group g's word lref with entry distance lf; true when any hit is done
+        // `leaves` leading leaves, lane group g's word lref with entry distance lf; true when any hit is
+        // done. A leaf is entered once, with the rayLength of that moment: a block of several passes of
+        // eight lanes (always alone) is not tested against its own hits, which rounding can place before
+        // its box. Leaves that are tested together take one pass each and are entered in order below.
         auto test_leaves = [&](uint32_t lref, float lf, unsigned leaves) {
             const unsigned g = lane >> 3, gl = lane & 7u;
+            const bool enter = lf <= wlen;
             const uint32_t k0 = g < leaves ? (lref & LEAF_BLOCK_MASK) * s.leafSize : 0u;
             const uint32_t cnt = g < leaves ? leaf_slots(s, lref, err) : 0u;
             for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
@@ -1013,7 +1017,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
                     ok = TRI ? intersect_triangle_wt_v(o, wt, a, b, c, h, hu, hv)
                              : intersect_triangle_v(o, d, a, b, c, h, hu, hv);
-                    ok = ok && h < wlen && lf <= wlen;
+                    ok = ok && enter && h < wlen;
                 }
                 if (!__any_sync(0xffffffffu, ok)) continue;
                 if (ANY_HIT) {
@@ -1030,7 +1034,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     if (!gm) continue;
                     const unsigned win = 8 * k + (unsigned)__ffs(gm) - 1;
                     const float kf = __shfl_sync(0xffffffffu, lf, win), kh = __shfl_sync(0xffffffffu, h, win);
-                    if (kf <= wlen && kh < wlen) {
+                    if ((leaves == 1 || kf <= wlen) && kh < wlen) {
                         wlen = kh;
                         wu = __shfl_sync(0xffffffffu, hu, win);
                         wv = __shfl_sync(0xffffffffu, hv, win);

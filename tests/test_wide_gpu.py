@@ -237,3 +237,31 @@ def test_direct_and_queued_small_calls(ctx, n):
     torch.cuda.synchronize()
     same(({k: v.cpu().numpy() for k, v in out.items()}, occ.cpu().numpy()), want)
     ds.close()
+
+
+@pytest.mark.parametrize("watertight", [False, True])
+@pytest.mark.parametrize("leaf", [9, 16, 32])
+@pytest.mark.parametrize("n", [3001, 20001, 200001])
+def test_leaves_of_several_passes(ctx, n, leaf, watertight):
+    """Overlapping coplanar triangles, up to 32 in a leaf: rounding puts hits just before the leaf's flat
+    box, after which a closer one in a later pass of the same leaf still counts. A warp per ray (one
+    launch, and from a queue) and the last rays of a lane walk."""
+    r = np.random.default_rng(leaf)
+    k = 64  # clusters of `leaf` triangles, each in its own plane z = const
+    p = r.uniform(-1, 1, (k, leaf, 3, 3))
+    p[..., 2] = r.uniform(-0.4, 0.4, (k, 1, 1))
+    p += np.stack(np.meshgrid(4 * np.arange(8), 4 * np.arange(8), [0], indexing="ij"), -1).reshape(k, 1, 1, 3)
+    p = p.reshape(-1, 3).astype(np.float32)
+    t = np.concatenate([np.arange(len(p)).reshape(-1, 3), np.zeros((k * leaf, 1), int)], 1).astype(np.uint32)
+    b = bvh.build_bvh(p, t, method="sweep", leaf_size=leaf)
+    full = b.slots.reshape(-1, leaf, 4)
+    assert ((full[..., 0] != full[..., 1]).sum(1) > 8).any()
+    ds = ctx.upload_scene(b, p)
+    ds.set_triangle_test(watertight)
+    at = r.integers(0, k, n)
+    target = p.reshape(k, -1, 3)[at].mean(1) + np.concatenate([r.uniform(-0.6, 0.6, (n, 2)), np.zeros((n, 1))], 1)
+    o = target + np.concatenate([r.uniform(-1, 1, (n, 2)), r.uniform(1, 3, (n, 1)) * r.choice([-1, 1], (n, 1))], 1)
+    d = target - o
+    rays = make_rays(o, d / np.linalg.norm(d, axis=1, keepdims=True), np.full(n, np.inf))
+    same(*both_modes(ctx, ds, rays))
+    ds.close()
