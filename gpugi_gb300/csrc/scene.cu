@@ -362,3 +362,9 @@ extern "C" gpugi_status gpugi_debug_limit_nodes(gpugi_scene* sc, uint32_t numNod
     sc->dev.wide = sc->dev.numNodes == sc->numNodesUploaded ? sc->wide : nullptr;
     return GPUGI_OK;
 }
+
+extern "C" gpugi_status gpugi_debug_wide_nodes(const gpugi_scene* sc, uint32_t* numNodes) {
+    if (!sc || !numNodes) return GPUGI_ERROR_INVALID_ARGUMENT;
+    *numNodes = sc->dev.wide ? sc->dev.numWide : 0u;
+    return GPUGI_OK;
+}

@@ -57,6 +57,7 @@ def _declare(L):
     L.gpugi_scene_destroy.restype = None
     L.gpugi_debug_raise_device_error.argtypes = [P, U32]
     L.gpugi_debug_limit_nodes.argtypes = [P, U32]
+    L.gpugi_debug_wide_nodes.argtypes = [P, C.POINTER(U32)]
     L.gpugi_set_async_walker_share.argtypes = [P, U32]
     L.gpugi_nrc_debug_stall.argtypes = [P, P, U32, U64]
     L.gpugi_scene_build.argtypes = [P, P, U32, P, U32, P, P, U32, U32, C.POINTER(P)]
@@ -251,6 +252,12 @@ class DeviceScene:
         parents[hier[left, 7].view(np.uint32)] = inner
         return B.BVH(hierarchy=hier, slots=slots, parents=parents, leaf_size=self.leaf_size, bounds_kind=self.bounds_kind,
                      max_depth=0)
+
+    def wide_nodes(self) -> int:
+        """Test support: nodes of the four-wide copy that trace mode 3 walks (0: the scene has none)."""
+        n = C.c_uint32()
+        self.ctx.check(lib().gpugi_debug_wide_nodes(self._h, C.byref(n)))
+        return n.value
 
     def set_triangle_test(self, watertight: bool) -> None:
         """Triangle test of the ray queries on this scene: the reference's

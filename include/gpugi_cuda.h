@@ -123,6 +123,9 @@ void gpugi_scene_destroy(gpugi_scene* scene);
  * reach a node at or past the limit end, and the checked library
  * (libgpugi_cuda_checked.so) reports GPUGI_DEVERR_BOUNDS for them. */
 gpugi_status gpugi_debug_limit_nodes(gpugi_scene* scene, uint32_t numNodes);
+/* Test support: the number of nodes of the scene's four-wide copy that trace
+ * mode 3 walks, 0 where the scene has none (gpugi_set_trace_config). */
+gpugi_status gpugi_debug_wide_nodes(const gpugi_scene* scene, uint32_t* numNodes);
 
 /* Build the hierarchy on the GPU and create the scene. Replaces a host
  * build with bvhmake (BVHBuilder::BuildBVH + FitBox + ExportBVH/

@@ -265,3 +265,102 @@ def test_leaves_of_several_passes(ctx, n, leaf, watertight):
     rays = make_rays(o, d / np.linalg.norm(d, axis=1, keepdims=True), np.full(n, np.inf))
     same(*both_modes(ctx, ds, rays))
     ds.close()
+
+
+def entering_rays(pos, tri, n, seed):
+    """Rays at triangles from outside: every one enters the scene's root bounds, so it is queued."""
+    r = np.random.default_rng(seed)
+    target = pos[tri[r.integers(0, len(tri), n), :3].astype(np.int64)].astype(np.float64).mean(1)
+    d = r.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    return make_rays(target - d * np.linalg.norm(np.ptp(pos, axis=0)), d, np.full(n, np.inf))
+
+
+@pytest.mark.parametrize("name", ["grid", "icosphere", "soup"])
+def test_scenes_have_a_wide_copy(ctx, name):
+    """The other tests compare modes, which agree whichever walker serves mode 3: here it is seen that
+    the builders' trees have the wide copy, with at most one wide node per inner node and the numbers
+    that the root's block of 256 leaves unused."""
+    pos, tri = SCENES[name]()
+    made = [ctx.upload_scene(bvh.build_bvh(pos, tri, method=m, leaf_size=leaf), pos)
+            for m, leaf in (("sweep", 1), ("sweep", 8), ("sweep", 32), ("kdtree", 8))]
+    for ds in made + [ctx.build_scene(pos, tri)]:
+        inner = (ds.num_nodes - 1) // 2
+        assert (inner - 1) // 3 <= ds.wide_nodes() <= inner + 256
+        ds.close()
+    two = ctx.upload_scene(bvh.build_bvh(*SCENES["two"](), method="sweep", leaf_size=2), SCENES["two"]()[0])
+    assert two.num_nodes == 1 and two.wide_nodes() == 0
+    two.close()
+    ds = ctx.upload_scene(bvh.build_bvh(pos, tri, method="sweep", fit="ellipsoid"), pos)
+    assert ds.wide_nodes() == 0
+    ds.close()
+
+
+@pytest.mark.parametrize("broken", ["not nested", "empty box", "nan box", "escape"])
+def test_broken_trees_have_no_wide_copy(ctx, broken):
+    s = scenes.displaced_icosphere(2048, seed=7)
+    b = bvh.build_bvh(s["positions"], s["triangles"], method="sweep", leaf_size=8)
+    ok = ctx.upload_scene(b, s["positions"])
+    assert ok.wide_nodes() > 0
+    ok.close()
+    h = b.hierarchy.copy()
+    word = h[:, 3].view(np.uint32)
+    inner = np.nonzero((word & 0x80000000) == 0)[0]
+    for i in (inner[0], inner[len(inner) // 3], inner[-1]):
+        g = h.copy()
+        if broken == "not nested":  # one child sticks out by one float
+            left = word[i]
+            g[left, 4] = np.nextafter(g[i, 4], np.float32(np.inf))
+        elif broken == "empty box":
+            g[word[i], [0, 4]] = [g[i, 4], g[i, 0]]
+        elif broken == "nan box":
+            g[word[i], 5] = np.nan
+        else:
+            left = word[i]
+            g[left, 7] = g[g[left, 7].view(np.uint32), 7]
+        b.hierarchy = g
+        ds = ctx.upload_scene(b, s["positions"])
+        assert ds.wide_nodes() == 0, i
+        ds.close()
+
+
+@pytest.mark.parametrize("inner", [71, 72, 73, 100])
+def test_chains_at_the_depth_limit(ctx, inner):
+    """A chain of inner nodes, each with one leaf: three of them per wide level, so 72 are the 24 levels
+    that the walk's stack holds and 73 keep the binary walkers. Boxes that all overlap fill the stack."""
+    r = np.random.default_rng(inner)
+    p = r.uniform(-1, 1, (inner + 1, 3, 3)).astype(np.float32)
+    lo, hi = p.min(1), p.max(1)
+    h = np.zeros((2 * inner + 1, 8), np.float32)
+    for k in range(inner + 1):
+        leaf = 2 * k + 1 if k < inner else 2 * inner
+        h[leaf, 0:3], h[leaf, 4:7] = lo[k], hi[k]
+        h[leaf, 3] = np.uint32(0x80000000 | k).view(np.float32)
+        h[leaf, 7] = np.uint32(2 * k + 2 if k < inner else 0).view(np.float32)
+        if k < inner:
+            h[2 * k, 0:3], h[2 * k, 4:7] = lo[k:].min(0), hi[k:].max(0)
+            h[2 * k, 3] = np.uint32(2 * k + 1).view(np.float32)  # its escape is 0: the last child of the last child
+    slots = np.concatenate([np.arange(3 * (inner + 1)).reshape(-1, 3), np.zeros((inner + 1, 1), int)], 1).astype(np.int32)
+    pos = p.reshape(-1, 3)
+    b = bvh.build_bvh(pos, slots.astype(np.uint32), method="sweep", leaf_size=1)
+    b.hierarchy, b.slots = h, slots
+    ds = ctx.upload_scene(b, pos)
+    assert (ds.wide_nodes() > 0) == (inner <= 72)
+    for n in (999, 30001):
+        same(*both_modes(ctx, ds, entering_rays(pos, slots, n, n)))
+    ds.close()
+
+
+@pytest.mark.parametrize("per_warp", [2, 5, 8, 32])
+def test_rules_on_rays_per_warp(ctx, per_warp):
+    """Both sides of each rule on the queue's length in rays per warp of the full grid (eight blocks of
+    four warps per SM): one launch without a queue up to 2, whole warps up to 5 (any hit) and 8
+    (closest hit), one ray per lane up to 32."""
+    import torch
+    s = scenes.displaced_icosphere(16384, seed=4)
+    ds = ctx.build_scene(s["positions"], s["triangles"])
+    assert ds.wide_nodes() > 0
+    at = per_warp * 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (at, at + 1):
+        same(*both_modes(ctx, ds, entering_rays(s["positions"], s["triangles"], n, n)))
+    ds.close()
