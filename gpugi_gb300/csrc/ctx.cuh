@@ -104,7 +104,7 @@ struct gpugi_scene {
     std::vector<int32_t> hostSlots;
     std::vector<float> hostMaterials;
     uint32_t numLeafBlocks = 0;
-    const float4* wide = nullptr;  // dev.wide before gpugi_debug_limit_nodes
+    uint32_t numWide = 0;  // dev.numWide before gpugi_debug_limit_nodes
     uint32_t numNodesUploaded = 0;  // dev.numNodes before gpugi_debug_limit_nodes
     // light tables (Scene::LoadLightSources / ComputePointLightTable)
     bool lightsReady = false;

@@ -3,6 +3,7 @@
 //
 // Replaces Scene::UploadGeometry / UploadHierarchy (gpugi/scene/scene.cpp:
 // 75-130) for the CUDA path.
+#include <algorithm>
 #include <cstring>
 
 #include "ctx.cuh"
@@ -358,8 +359,9 @@ extern "C" gpugi_status gpugi_debug_limit_nodes(gpugi_scene* sc, uint32_t numNod
     if (numNodes > sc->numNodesUploaded)
         return fail(sc->ctx, GPUGI_ERROR_INVALID_ARGUMENT, "the node limit can only be lowered");
     sc->dev.numNodes = numNodes ? numNodes : sc->numNodesUploaded;
-    // the wide copy holds every node: a lowered limit is walked on the binary tree
-    sc->dev.wide = sc->dev.numNodes == sc->numNodesUploaded ? sc->wide : nullptr;
+    // the wide copy's limit is lowered in proportion
+    if (sc->dev.wide)
+        sc->dev.numWide = std::max<uint32_t>(1u, (uint64_t)sc->numWide * sc->dev.numNodes / sc->numNodesUploaded);
     return GPUGI_OK;
 }
 

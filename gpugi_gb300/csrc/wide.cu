@@ -180,7 +180,7 @@ __global__ void k_wide_fill(const float4* __restrict__ nodes, uint32_t n, const 
 
 gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc) {
     sc->dev.wide = nullptr;
-    sc->dev.numWide = 0;
+    sc->numWide = sc->dev.numWide = 0;
     const uint32_t n = sc->dev.numNodes;
     if (sc->dev.boundsKind != GPUGI_BOUNDS_AABB || sc->dev.topNodes || n < 3) return GPUGI_OK;
     cudaStream_t st = ctx->stream;
@@ -220,8 +220,8 @@ gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc) {
     const uint32_t numbers = 256 + ~got[2];  // the root's block leaves some of its numbers unused
     const bool fits = ~got[1] + 1 <= kMaxLevels && numbers < (1u << 25);
     if (got[0] == 0 || !fits || numbers > count) return GPUGI_OK;
-    sc->wide = sc->dev.wide = wide;
-    sc->dev.numWide = numbers;
+    sc->dev.wide = wide;
+    sc->numWide = sc->dev.numWide = numbers;
     return GPUGI_OK;
 }
 

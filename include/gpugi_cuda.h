@@ -118,13 +118,15 @@ gpugi_status gpugi_scene_upload(gpugi_ctx* ctx, const float* hierarchy, uint32_t
                                 uint32_t numMaterials, gpugi_scene** out);
 void gpugi_scene_destroy(gpugi_scene* scene);
 /* Test support: the node count the device code checks indexes against is
- * lowered to numNodes (at most the scene's own; 0 restores it). The node
- * array itself is unchanged, so every fetch stays inside it; walks that
- * reach a node at or past the limit end, and the checked library
- * (libgpugi_cuda_checked.so) reports GPUGI_DEVERR_BOUNDS for them. */
+ * lowered to numNodes (at most the scene's own; 0 restores it), and that of
+ * the four-wide copy in proportion. The node arrays themselves are unchanged,
+ * so every fetch stays inside them; walks that reach a node at or past the
+ * limit end (a warp that walks one ray leaves the node out), and the checked
+ * library (libgpugi_cuda_checked.so) reports GPUGI_DEVERR_BOUNDS for them. */
 gpugi_status gpugi_debug_limit_nodes(gpugi_scene* scene, uint32_t numNodes);
-/* Test support: the number of nodes of the scene's four-wide copy that trace
- * mode 3 walks, 0 where the scene has none (gpugi_set_trace_config). */
+/* Test support: the node count of the scene's four-wide copy, which trace mode
+ * 3 walks, as the device code checks it; 0 where the scene has none
+ * (gpugi_set_trace_config). */
 gpugi_status gpugi_debug_wide_nodes(const gpugi_scene* scene, uint32_t* numNodes);
 
 /* Build the hierarchy on the GPU and create the scene. Replaces a host

@@ -91,3 +91,75 @@ def test_checked_library(tmp_path):
                        timeout=900)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
     assert "checked library ok" in r.stdout
+
+
+WIDE_CHILD = r'''
+import re
+
+import torch
+
+from gpugi_gb300 import bvh, cuda, render, scenes
+
+L = cuda.lib()
+assert L.gpugi_version().endswith(b"checked"), L.gpugi_version()
+ctx = cuda.Context()
+sc = scenes.cornell_room(seed=1, sphere_level=3, wall_grid=20)
+b = bvh.build_bvh(sc["positions"], sc["triangles"], method="sweep")
+ds = ctx.upload_scene(b, sc["positions"], cuda.vertex_info(sc["normals"], sc["texcoords"]), sc["materials"])
+full = ds.wide_nodes()
+warps = 32 * torch.cuda.get_device_properties(0).multi_processor_count  # of the full grid
+
+
+def raises(f):
+    try:
+        f()
+    except cuda.GpugiError as e:
+        m = re.search(r"error bits (0x[0-9a-f]+)", str(e))
+        return e.status == 5 and bool(m) and int(m.group(1), 16) & 0x20 != 0
+    return False
+
+
+# whole warps from the caller's arrays and from a queue, a lane per ray, the passes' and batches' walkers
+calls = []
+for n in (1000, 4 * warps, 16 * warps):
+    rays = scenes.aimed_rays(n, sc["positions"], seed=n)
+    calls += [lambda r=rays: cuda.trace_closest(ctx, ds, r), lambda r=rays: cuda.trace_any(ctx, ds, r)]
+cam = render.camera_lookat(*scenes.CORNELL_CAMERA, 96, 96)
+img = render.Image(ctx, 96, 96)
+
+
+def frame():
+    render.render(ctx, ds, cam, img, "PT", max_path_length=4, samples=2, rng_state=[3])
+    ctx.sync()
+
+
+def batch():
+    render.render_batch(ctx, [dict(scene=ds, camera=cam, image=img, pass_="PT", samples=2, max_path_length=4,
+                                   rng_state=[3])])
+    ctx.sync()
+
+
+calls += [frame, batch]
+for wt in (False, True):
+    ds.set_triangle_test(wt)
+    for limit in (0, b.num_nodes // 2, 0):
+        ctx.check(L.gpugi_debug_limit_nodes(ds.handle, limit))
+        assert ds.wide_nodes() == (full * limit // b.num_nodes if limit else full) > 0
+        for k, call in enumerate(calls):
+            assert raises(call) == (limit != 0), (wt, limit, k)
+            assert ctx.device_error_bits() == 0
+ds.close()
+print("checked library ok")
+'''
+
+
+@pytest.mark.gpu
+def test_checked_wide_walkers(tmp_path):
+    """The wide walkers' own node checks, as above: the scene keeps its wide copy under a lowered limit,
+    and every kind of walk over it reports the bounds bit."""
+    script = tmp_path / "checked_wide_child.py"
+    script.write_text(WIDE_CHILD)
+    env = dict(os.environ, GPUGI_CHECKED="1", PYTHONPATH=str(ROOT))
+    r = subprocess.run([sys.executable, str(script)], cwd=ROOT, env=env, capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-3000:]
+    assert "checked library ok" in r.stdout
