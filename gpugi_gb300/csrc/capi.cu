@@ -200,17 +200,23 @@ static bool ensure_bounce(gpugi_ctx* ctx) {
 }
 
 // Ray queries on host arrays. Rays go through device staging in chunks of at
-// most 2^22. With trace modes 2-5 a chunk of page-locked arrays is split into
-// ctx->hostParts parts whose copies in (copyIn stream), traversal (the context
-// stream and a second one, alternating by part) and copies out (copyOut
-// stream) overlap: part p+1 uploads while part p is traced, part p downloads
-// while part p+1 is traced, and the traversals of neighbouring parts overlap
-// too. Each part has its own queue range and counters. Copies of pageable
-// memory keep the host waiting and overlap with next to nothing, so such
-// arrays stay in one part (aimed rays at the icosphere of 65k triangles, one /
-// two parts: 300k rays 436 / 528 us, 2^20 1.26 / 1.32 ms, 2^22 4.46 / 4.39 ms;
-// page-locked 2^20 1.16 / 1.09 ms, 2^22 4.28 / 3.87 ms). Returns when every
-// result is in host memory.
+// most 2^22. With trace modes 2-5 a chunk is split into ctx->hostParts parts
+// whose copies in (copyIn stream), traversal (the context stream and a second
+// one, alternating by part) and copies out (copyOut stream) overlap: part p+1
+// uploads while part p is traced, part p downloads while part p+1 is traced,
+// and the traversals of neighbouring parts overlap too. Each part has its own
+// queue range and counters. Returns when every result is in host memory.
+// Copies of pageable memory keep the host waiting and overlap with little, so
+// chunks below kPagedParts rays stay in one part where the rays or the results
+// are pageable. Aimed rays at the icosphere of 65k triangles, one / two parts,
+// in us (rays, results):
+//                          300k          2^20           2^22
+//   pageable, pageable     448 / 487     1,202 / 1,198  4,394 / 4,266
+//   page-locked, pageable  437 / 457     1,165 / 1,090  4,299 / 3,884
+//   pageable, page-locked  438 / 478     1,169 / 1,169  4,388 / 4,257
+//   page-locked, both      432 / 452     1,156 / 1,084  4,286 / 3,878
+//   managed, both          1,426 / 1,338 3,611 / 3,278  16,305 / 14,439
+constexpr uint64_t kPagedParts = 1ull << 20;
 static gpugi_status trace_host(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* const src[7],
                                uint64_t n, int32_t* slot, float* t, float* u, float* v, uint8_t* occ) {
     // Page-locked arrays: the kernels read the rays and write the results
@@ -262,7 +268,8 @@ static gpugi_status trace_host(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHi
     uint8_t* dOcc = reinterpret_cast<uint8_t*>(base + 7 * col);
     char* const dRes[4] = {base + 7 * col, base + 8 * col, base + 9 * col, base + 10 * col};
     const uint32_t parts = std::min<uint32_t>(std::max<uint32_t>(ctx->hostParts, 1u), 8u);
-    const bool pipe = ctx->traceMode >= 2 && parts > 1 && chunk >= (1ull << 16) && mapped_host(src[0]) && mapped_host(outs[0]);
+    const bool pipe = ctx->traceMode >= 2 && parts > 1 && chunk >= (1ull << 16) &&
+                      (chunk >= kPagedParts || !(plain_host(src[0]) || plain_host(outs[0])));
     if (pipe) {
         if ((st = ensure_pipeline(ctx)) || (st = ensure_queue(ctx, chunk))) return st;
     }

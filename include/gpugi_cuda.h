@@ -313,12 +313,12 @@ gpugi_status gpugi_set_trace_config(gpugi_ctx* ctx, uint32_t mode, uint32_t bloc
 
 /* Host-pointer ray queries (gpugi_trace_closest / gpugi_trace_any). The
  * arrays go through device staging, small pageable ones through a page-locked
- * block of the context that the kernels work on over the host link. Calls on
- * page-locked arrays (cudaHostAlloc, cudaHostRegister) are split into `parts`
- * parts (1-8, default 2) whose copies to the device, traversal and copies
- * back overlap on separate streams (trace modes 2-5; neighbouring parts are
- * traversed on two streams, so one part's walker tail overlaps the next
- * part's walk; 1 disables the overlap). With zeroCopy (default 0) and every
+ * block of the context that the kernels work on over the host link. Calls of
+ * 2^16 rays and more (2^20 where the rays or the results are in pageable
+ * memory) are split into `parts` parts (1-8, default 2) whose copies to the
+ * device, traversal and copies back overlap on separate streams (trace modes
+ * 2-5; neighbouring parts are traversed on two streams, so one part's walker
+ * tail overlaps the next part's walk; 1 disables the overlap). With zeroCopy (default 0) and every
  * array page-locked, the kernels instead read the rays and write the results
  * over the host link directly, in one part. Results are the same on every
  * path. */

@@ -543,3 +543,51 @@ def test_host_arrays_of_each_size(cuda_ctx, icosphere_65536, n, shift):
         np.testing.assert_array_equal(got[k].view(np.uint32), want[k].cpu().numpy().view(np.uint32), err_msg=k)
     np.testing.assert_array_equal(got_occ, occ.cpu().numpy())
     ds.close()
+
+
+@pytest.mark.parametrize("kinds", ["pageable", "managed", "locked rays", "locked results"])
+@pytest.mark.parametrize("n", [1000, 65537, (1 << 20) - 1, (1 << 20) + 1])
+def test_host_arrays_of_each_kind(cuda_ctx, icosphere_65536, n, kinds):
+    """Rays and results in pageable, page-locked and managed memory, on both sides of the sizes from
+    which calls are split into parts: the device arrays' results, bit for bit."""
+    import ctypes
+
+    import torch
+    sc = icosphere_65536
+    ds = cuda_ctx.build_scene(sc["positions"], sc["triangles"])
+    torch.cuda.synchronize()
+    owned = []
+
+    def managed(shape):
+        rt = ctypes.CDLL("libcudart.so.13")  # the runtime that torch has loaded
+        p, count = ctypes.c_void_p(), int(np.prod(shape))
+        assert rt.cudaMallocManaged(ctypes.byref(p), ctypes.c_size_t(4 * count), 1) == 0
+        owned.append((rt, p))
+        return np.ctypeslib.as_array(ctypes.cast(p, ctypes.POINTER(ctypes.c_float)), shape=(count,)).reshape(shape)
+
+    plain = lambda shape: np.zeros(shape, np.float32)  # noqa: E731
+    locked = lambda shape: torch.empty(shape, dtype=torch.float32).pin_memory().numpy()  # noqa: E731
+    src, dst = {"pageable": (plain, plain), "managed": (managed, managed), "locked rays": (locked, plain),
+                "locked results": (plain, locked)}[kinds]
+    host = scenes.aimed_rays(n, sc["positions"], seed=n, spread=2.5)
+    rays, res = src((7, n)), dst((5, n))
+    for k, key in enumerate(cuda.RAY_KEYS):
+        rays[k] = host[key]
+    dev = {k: torch.from_numpy(host[k]).cuda() for k in cuda.RAY_KEYS}
+    want = {k: torch.empty(n, dtype=torch.int32 if k == "slot" else torch.float32, device="cuda")
+            for k in ("slot", "t", "u", "v")}
+    occ = torch.empty(n, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    cuda.trace_closest_device(cuda_ctx, ds, dev, want)
+    cuda.trace_any_device(cuda_ctx, ds, dev, occ)
+    cuda_ctx.sync()
+    lib, args = cuda.lib(), [cuda._ptr(rays[k]) for k in range(7)]
+    cuda_ctx.check(lib.gpugi_trace_closest(cuda_ctx.handle, ds.handle, *args, n, *[cuda._ptr(res[k]) for k in range(4)]))
+    cuda_ctx.check(lib.gpugi_trace_any(cuda_ctx.handle, ds.handle, *args, n, cuda._ptr(res[4])))
+    for k, key in enumerate(("slot", "t", "u", "v")):
+        np.testing.assert_array_equal(res[k].view(np.uint32), want[key].cpu().numpy().view(np.uint32), err_msg=key)
+    np.testing.assert_array_equal(res[4].view(np.uint8)[:n], occ.cpu().numpy())
+    ds.close()
+    del rays, res
+    for rt, p in owned:
+        assert rt.cudaFree(p) == 0
