@@ -33,6 +33,7 @@ namespace gpugi {
 namespace {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu;  // no child, no index
+constexpr size_t kKeptScratch = 16u << 20;  // 838,000 nodes
 constexpr uint32_t kMaxLevels = kWideStack / 3;  // a walk's stack holds at most three entries per wide level
 
 // kids[i]: the children (binary node indexes, increasing, kNone behind the
@@ -184,45 +185,65 @@ gpugi_status build_wide(gpugi_ctx* ctx, gpugi_scene* sc) {
     const uint32_t n = sc->dev.numNodes;
     if (sc->dev.boundsKind != GPUGI_BOUNDS_AABB || sc->dev.topNodes || n < 3) return GPUGI_OK;
     cudaStream_t st = ctx->stream;
-    // scratch in the context's staging buffer (kept between calls; every user of it finishes before it
-    // returns): {checks passed, ~deepest level, ~nodes behind block 0's}, children, index
-    if (gpugi_status gs = ensure_stage(ctx, 256 + 20 * (size_t)n)) {
-        cudaGetLastError();
-        return gs == GPUGI_ERROR_OUT_OF_MEMORY ? GPUGI_OK : gs;  // the binary walkers need no extra memory
-    }
-    uint32_t* word = static_cast<uint32_t*>(ctx->stageDev);
-    uint4* kids = reinterpret_cast<uint4*>(static_cast<char*>(ctx->stageDev) + 256);
-    uint32_t* index = reinterpret_cast<uint32_t*>(kids + n);
-    const unsigned grid = (n + 255) / 256;
-    GPUGI_CUDA_TRY(ctx, cudaMemsetAsync(word, 0xFF, 12, st));
-    k_wide_kids<<<grid, 256, 0, st>>>(sc->dev.nodes, n, kids, word);
-    k_wide_mark<<<grid, 256, 0, st>>>(kids, n, index, word + 1, word + 2);
-    // At most every inner node is a wide one: small trees allocate for that (64 B a node), so that the
-    // host waits once; large ones read the count first.
-    uint32_t got[3], count = 256 + (n - 1) / 2;
-    if (n > (1u << 20)) {
-        GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got, word, 12, cudaMemcpyDeviceToHost, st));
-        GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-        if (~got[2] > (n - 1) / 2) return GPUGI_OK;
-        count = 256 + ~got[2];
-    }
-    float4* wide = nullptr;
-    if (cudaMalloc(&wide, 128 * (size_t)count) != cudaSuccess) {
+    // Scratch: {checks passed, ~deepest level, ~nodes behind block 0's}, children, index. Up to
+    // kKeptScratch it is the context's staging buffer, which is kept between calls (every user of it
+    // finishes before it returns) and which host-array queries make as large; above, it goes again with
+    // this call. No memory for it or for the copy: the binary walkers need none.
+    const size_t scratchBytes = 256 + 20 * (size_t)n;
+    void *own = nullptr, *wide = nullptr;
+    if (scratchBytes <= kKeptScratch) {
+        if (gpugi_status gs = ensure_stage(ctx, scratchBytes)) {
+            cudaGetLastError();
+            return gs == GPUGI_ERROR_OUT_OF_MEMORY ? GPUGI_OK : gs;
+        }
+    } else if (cudaMalloc(&own, scratchBytes) != cudaSuccess) {
         cudaGetLastError();
         return GPUGI_OK;
     }
-    sc->allocations.push_back(wide);
-    k_wide_fill<<<grid, 256, 0, st>>>(sc->dev.nodes, n, kids, index, count, wide, word);
-    GPUGI_CUDA_TRY(ctx, cudaGetLastError());
-    GPUGI_CUDA_TRY(ctx, cudaMemcpyAsync(got, word, 12, cudaMemcpyDeviceToHost, st));
-    GPUGI_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    char* scratch = static_cast<char*>(own ? own : ctx->stageDev);
+    uint32_t* word = reinterpret_cast<uint32_t*>(scratch);
+    uint4* kids = reinterpret_cast<uint4*>(scratch + 256);
+    uint32_t* index = reinterpret_cast<uint32_t*>(kids + n);
+    auto leave = [&](gpugi_status gs) {  // what the scene does not keep (its stream has been waited for, or failed)
+        if (own) cudaFree(own);
+        if (wide && !sc->dev.wide) cudaFree(wide);
+        return gs;
+    };
+    auto check = [&](cudaError_t e) { return e == cudaSuccess ? GPUGI_OK : cuda_fail(ctx, e, "wide hierarchy"); };
+    const unsigned grid = (n + 255) / 256;
+    gpugi_status gs = check(cudaMemsetAsync(word, 0xFF, 12, st));
+    if (gs) return leave(gs);
+    k_wide_kids<<<grid, 256, 0, st>>>(sc->dev.nodes, n, kids, word);
+    k_wide_mark<<<grid, 256, 0, st>>>(kids, n, index, word + 1, word + 2);
+    uint32_t got[3];
+    auto read = [&]() {
+        if (gpugi_status e = check(cudaMemcpyAsync(got, word, 12, cudaMemcpyDeviceToHost, st))) return e;
+        return check(cudaStreamSynchronize(st));
+    };
+    // At most every inner node is a wide one: small trees allocate for that (64 B a node, 4 MiB), so that
+    // the host waits once; large ones read the count first.
+    uint32_t count = 256 + (n - 1) / 2;
+    if (n > (1u << 16)) {
+        if ((gs = read())) return leave(gs);
+        if (got[0] == 0 || ~got[2] > (n - 1) / 2) return leave(GPUGI_OK);
+        count = 256 + ~got[2];
+    }
+    if (cudaMalloc(&wide, 128 * (size_t)count) != cudaSuccess) {
+        cudaGetLastError();
+        wide = nullptr;
+        cudaStreamSynchronize(st);
+        return leave(GPUGI_OK);
+    }
+    k_wide_fill<<<grid, 256, 0, st>>>(sc->dev.nodes, n, kids, index, count, static_cast<float4*>(wide), word);
+    if ((gs = check(cudaGetLastError())) || (gs = read())) return leave(gs);
     // a walk's stack holds at most three entries per wide level, and its node offsets are 32-bit bytes
     const uint32_t numbers = 256 + ~got[2];  // the root's block leaves some of its numbers unused
     const bool fits = ~got[1] + 1 <= kMaxLevels && numbers < (1u << 25);
-    if (got[0] == 0 || !fits || numbers > count) return GPUGI_OK;
-    sc->dev.wide = wide;
+    if (got[0] == 0 || !fits || numbers > count) return leave(GPUGI_OK);
+    sc->allocations.push_back(wide);
+    sc->dev.wide = static_cast<const float4*>(wide);
     sc->numWide = sc->dev.numWide = numbers;
-    return GPUGI_OK;
+    return leave(GPUGI_OK);
 }
 
 }  // namespace gpugi

@@ -364,3 +364,45 @@ def test_rules_on_rays_per_warp(ctx, per_warp):
     for n in (at, at + 1):
         same(*both_modes(ctx, ds, entering_rays(s["positions"], s["triangles"], n, n)))
     ds.close()
+
+
+def test_memory_of_the_wide_copy():
+    """Trees of a million nodes, where the copy's upper bound (64 B a node) and its scratch (20 B) are
+    tens of megabytes: an accepted scene holds 128 B per wide node beside its arrays, one that fails the
+    checks nothing, and no scratch stays behind. 8 MiB of slack for the allocator's rounding."""
+    import torch
+    mib = 1 << 20
+    s = scenes.heightfield_boxes(seed=1, grid=500)
+    pos, tri = s["positions"], s["triangles"]
+    c = cuda.Context(0)
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info(0)[0]
+
+    first = c.build_scene(pos, tri, leaf_size=1)  # modules and the builder's own buffers are loaded
+    b = first.export()
+    first.close()
+    before = free()
+    arrays = 32 * len(b.hierarchy) + (16 + 48) * len(b.slots) + 12 * len(pos)
+    assert len(b.hierarchy) > 1_000_000
+    ds = c.upload_scene(b, pos)
+    wide = ds.wide_nodes()
+    assert wide > 0 and before - free() <= arrays + 128 * wide + 8 * mib
+    ds.close()
+    assert before - free() <= 8 * mib
+    b.hierarchy[b.hierarchy[0, 3].view(np.uint32), 4] = np.nextafter(b.hierarchy[0, 4], np.float32(np.inf))
+    ds = c.upload_scene(b, pos)
+    assert ds.wide_nodes() == 0 and before - free() <= arrays + 8 * mib
+    ds.close()
+    c.close()
+    # the scratch of a build goes with the call
+    c = cuda.Context(0)
+    small = c.build_scene(pos, tri[:1000], leaf_size=1)
+    before = free()
+    ds = c.build_scene(pos, tri, leaf_size=1)
+    assert ds.wide_nodes() > 0
+    ds.close()
+    assert before - free() <= 8 * mib
+    small.close()
+    c.close()
