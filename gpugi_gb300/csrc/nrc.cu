@@ -158,7 +158,7 @@ GPUGI_D void encode_tile(const float* __restrict__ records, int stride, uint64_t
     const int lane = threadIdx.x & 31;
     if (lane < 16) {
         const uint64_t i = base + lane;
-        __half row[kIn];
+        __align__(16) __half row[kIn];
         if (i < n) {
             const float* p = records + (uint64_t)stride * i;
             Query q;
@@ -482,7 +482,7 @@ __global__ void k_nrc_encode(const float* __restrict__ queries, uint64_t n, floa
                              __half* __restrict__ out) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    __half row[kIn];
+    __align__(16) __half row[kIn];
     encode(load_query(queries, i), boxMin, boxInv, row);
     for (int k = 0; k < kIn; ++k) out[i * kIn + k] = row[k];
 }

@@ -33,46 +33,9 @@ struct Query {  // one cache lookup / training sample
     float3 pos, dir, normal, albedo;
 };
 
-// Frequency + spherical-harmonics encoding of one query into 64 halves.
-GPUGI_D void encode(const Query& q, float3 boxMin, float3 boxInvExtent, __half* out) {
-    const float p[3] = {(q.pos.x - boxMin.x) * boxInvExtent.x, (q.pos.y - boxMin.y) * boxInvExtent.y,
-                        (q.pos.z - boxMin.z) * boxInvExtent.z};
-    int k = 0;
-    for (int d = 0; d < 3; ++d) {
-        float f = kPI_F * p[d];
-#pragma unroll
-        for (int o = 0; o < 6; ++o) {
-            float s, c;
-            sincosf(f, &s, &c);
-            out[k++] = __float2half(s);
-            out[k++] = __float2half(c);
-            f *= 2.0f;
-        }
-    }
-    const float x = q.dir.x, y = q.dir.y, z = q.dir.z;
-    const float xx = x * x, yy = y * y, zz = z * z;
-    const float sh[16] = {0.28209479f,
-                          -0.48860251f * y, 0.48860251f * z, -0.48860251f * x,
-                          1.09254843f * x * y, -1.09254843f * y * z, 0.31539157f * (3.0f * zz - 1.0f),
-                          -1.09254843f * x * z, 0.54627422f * (xx - yy),
-                          0.59004359f * y * (-3.0f * xx + yy), 2.89061144f * x * y * z,
-                          0.45704580f * y * (1.0f - 5.0f * zz), 0.37317633f * z * (5.0f * zz - 3.0f),
-                          0.45704580f * x * (1.0f - 5.0f * zz), 1.44530572f * z * (xx - yy),
-                          0.59004359f * x * (-xx + 3.0f * yy)};
-#pragma unroll
-    for (int i = 0; i < 16; ++i) out[k++] = __float2half(sh[i]);
-    out[k++] = __float2half(q.normal.x);
-    out[k++] = __float2half(q.normal.y);
-    out[k++] = __float2half(q.normal.z);
-    out[k++] = __float2half(q.albedo.x);
-    out[k++] = __float2half(q.albedo.y);
-    out[k++] = __float2half(q.albedo.z);
-    out[k++] = __float2half(1.0f);
-    while (k < kIn) out[k++] = __float2half(0.0f);
-}
-
-// The same encoding in 16-byte chunks of eight features (chunk c = features
-// [8 c, 8 c + 8)), for threads that share a query or store it chunk by chunk.
+// Frequency + spherical-harmonics encoding of one query, in 16-byte chunks of
+// eight features (chunk c = features [8 c, 8 c + 8)), so that threads can share a
+// query and store it chunk by chunk.
 struct EncodeInput {
     float f[3];    // pi x position in the box; octave o of an axis is f 2^o, exactly
     float sh[16];
@@ -119,6 +82,19 @@ GPUGI_D uint4 encode_chunk(const EncodeInput& e) {
         w[i] = *reinterpret_cast<uint32_t*>(&h);
     }
     return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// All chunks of a query; out is 16-byte aligned.
+GPUGI_D void encode(const Query& q, float3 boxMin, float3 boxInvExtent, __half* out) {
+    const EncodeInput e = encode_input(q, boxMin, boxInvExtent);
+    uint4* o = reinterpret_cast<uint4*>(out);
+    o[0] = encode_chunk<0>(e);
+    o[1] = encode_chunk<1>(e);
+    o[2] = encode_chunk<2>(e);
+    o[3] = encode_chunk<3>(e);
+    o[4] = encode_chunk<4>(e);
+    o[5] = encode_chunk<5>(e);
+    o[6] = encode_chunk<6>(e);
+    o[7] = encode_chunk<7>(e);
 }
 
 }  // namespace nrc
