@@ -406,3 +406,20 @@ def test_memory_of_the_wide_copy():
     assert before - free() <= 8 * mib
     small.close()
     c.close()
+
+
+@pytest.mark.parametrize("watertight", [False, True])
+@pytest.mark.parametrize("fit", ["ellipsoid", "obox"])
+def test_group_and_lane_rule(ctx, fit, watertight):
+    """Trees without a wide copy: queues on both sides of the rule between 8-lane groups and lanes (48
+    rays per block, eight blocks per SM: 58,368 on 152 SMs), every ray entering the scene."""
+    import torch
+    s = scenes.instanced_scene(seed=3, num_triangles=8000)
+    pos, tri = s["positions"], s["triangles"]
+    ds = ctx.upload_scene(bvh.build_bvh(pos, tri, method="sweep", fit=fit), pos)
+    ds.set_triangle_test(watertight)
+    assert ds.wide_nodes() == 0
+    at = 48 * 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (at - 1, at):
+        same(*both_modes(ctx, ds, entering_rays(pos, tri, n, n)))
+    ds.close()
