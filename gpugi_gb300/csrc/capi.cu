@@ -545,6 +545,13 @@ static gpugi_status stream_scratch(gpugi_ctx* ctx, cudaStream_t s, uint64_t n, g
     return GPUGI_OK;
 }
 
+// Streams that the context's last kMaxQueryStreams stream-ordered calls went to.
+static uint32_t streams_in_use(const gpugi_ctx* ctx) {
+    uint32_t k = 0;
+    for (const auto& e : ctx->streamScratch) k += e.tick + kMaxQueryStreams > ctx->streamTick ? 1u : 0u;
+    return k;
+}
+
 static gpugi_status trace_async(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* ox,
                                 const float* oy, const float* oz, const float* dx, const float* dy, const float* dz,
                                 const float* tmax, uint64_t n, int32_t* slot, float* t, float* u, float* v,
@@ -556,7 +563,7 @@ static gpugi_status trace_async(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyH
     gpugi_status st = stream_scratch(ctx, s, n, &ss);
     if (st) return st;
     st = launch_trace_filtered_on(ctx, sc, anyHit, ox, oy, oz, dx, dy, dz, tmax, n, slot, t, u, v, occluded,
-                                  ss->queue, ss->counters, s, ctx->asyncWalkerShare);
+                                  ss->queue, ss->counters, s, ctx->asyncWalkerShare, streams_in_use(ctx));
     if (st) return st;
     GPUGI_CUDA_TRY(ctx, cudaEventRecord(ss->lastUse, s));
     return GPUGI_OK;

@@ -474,14 +474,15 @@ gpugi_status launch_trace_filtered(gpugi_ctx* ctx, const gpugi_scene* sc, bool a
                                     ctx->queue, counters);
 }
 
-// The same two launches as launch_trace_filtered, on scratch memory the
-// caller provides (queue of n entries, 4 counters, which it zeroes on the
-// stream); allocates nothing.
+// The same launches as launch_trace_filtered, on scratch memory the caller
+// provides (queue of n entries, 4 counters, which it zeroes on the stream);
+// allocates nothing. streams: how many the caller's queries are spread over.
 gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* ox,
                                       const float* oy, const float* oz, const float* dx, const float* dy,
                                       const float* dz, const float* tmax, uint64_t n, int32_t* slot, float* t,
                                       float* u, float* v, uint8_t* occluded, uint32_t* queue,
-                                      unsigned long long* counters, cudaStream_t stream, uint32_t walkerShare) {
+                                      unsigned long long* counters, cudaStream_t stream, uint32_t walkerShare,
+                                      uint32_t streams) {
     if (n == 0) return GPUGI_OK;
     cudaStream_t cs = stream ? stream : ctx->stream;
     const int ell = (int)sc->dev.boundsKind;  // bounds kind: 0 box, 1 ellipsoid, 2 oriented box
@@ -537,10 +538,17 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
         WalkerLaunch L;
         gpugi_status st = walker_launch_config(ctx, sc, (const void*)kw, 1ull << 40, 0, L);
         if (st) return st;
-        // a share below 100 is a stream-ordered query beside others: the wide walker then takes 70 %
-        // of it again, since its lanes refill (8 batches of 2^20 rays over four streams, 66k of them
-        // entering the scene: 541 us at the share as it is, 487 at 80-70 %, 466 at 60 %, 530 at 50 %)
-        L.grid = share_of_grid(L.grid, walkerShare < 100 ? (walkerShare * 7 + 9) / 10 : 100);
+        // Queries on one or two streams launch the share each; on more they have 2.8 shares between
+        // them, but at least half of one: walkers beyond that wait for SMs, or hold them with idle lanes.
+        // Us a batch at 50 / 37 / 25 / 19 % of the grid (2^20 random rays at the 65k icosphere, 66k of
+        // which enter; 66k aimed ones; 2^20 aimed ones), 8 batches over 4 streams at 35 / 37.5 %: 441 / 450:
+        //   2 streams   79.0 / 86.1 / 95.0 / 108.6   88.4 / 97.4 / 113.1 / 132.0   854 / 998 / 1,305 / 1,625
+        //   3           59.7 / 63.6 / 69.3 / 77.9    68.0 / 71.8 / 82.3 / 94.7     837 / 843 / 983 / 1,185
+        //   4           58.8 / 55.1 / 56.5 / 62.5    66.3 / 62.3 / 67.4 / 75.8     836 / 837 / 844 / 974
+        //   6           59.2 / 54.5 / 49.6 / 50.2    65.9 / 61.6 / 58.9 / 58.9     837 / 837 / 836 / 853
+        //   8           59.5 / 54.5 / 53.1 / 52.7    66.0 / 61.8 / 61.7 / 63.6     836 / 837 / 839 / 888
+        const uint32_t tenths = std::min(std::max(10u * streams, 28u), 56u);
+        L.grid = std::max(1u, share_of_grid(L.grid, walkerShare) * 28u / tenths);
         kw<<<L.grid, 128, 0, cs>>>(sc->dev, ox, oy, oz, dx, dy, dz, tmax, slot, t, u, v, occluded, queue, counters,
                                    ctx->errWord);
         GPUGI_CUDA_TRY(ctx, cudaGetLastError());

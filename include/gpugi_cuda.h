@@ -326,10 +326,12 @@ gpugi_status gpugi_set_host_pipeline(gpugi_ctx* ctx, uint32_t parts, uint32_t ze
 /* Share (percent, 1-100, default 50) of the persistent walker grid that a
  * stream-ordered query on device arrays (gpugi_trace_*_device_async)
  * launches. Queries on several streams then walk side by side, each one's
- * tail of deep walks overlapping the others' bulk: on the 2^20-ray
- * closest-hit workload over 4 streams, 50 % gives ~7 % more rays/s than the
- * full grid. Synchronous calls and host-array queries (paced by their
- * copies) use the full grid; results do not depend on the share. */
+ * tail of deep walks overlapping the others' bulk. The walker of box
+ * hierarchies (trace mode 3) takes the share as it is while the context's
+ * last eight stream-ordered queries went to one or two streams; on more,
+ * queries have 2.8 shares between them, down to half a share each.
+ * Synchronous calls and host-array queries (paced by their copies) use the
+ * full grid; results do not depend on the share. */
 gpugi_status gpugi_set_async_walker_share(gpugi_ctx* ctx, uint32_t percent);
 
 /* Scene layout tuning (set by the autotuner), applied to scenes uploaded

@@ -423,3 +423,34 @@ def test_group_and_lane_rule(ctx, fit, watertight):
     for n in (at - 1, at):
         same(*both_modes(ctx, ds, entering_rays(pos, tri, n, n)))
     ds.close()
+
+
+@pytest.mark.parametrize("share", [1, 50, 99, 100])
+@pytest.mark.parametrize("streams", [1, 3, 4, 9])
+def test_shares_over_streams(ctx, streams, share):
+    """Stream-ordered walks on every grid that the share and the number of streams lead to, more streams
+    than the context has scratch sets for among them: the synchronous calls' results."""
+    import torch
+    s = scenes.displaced_icosphere(16384, seed=4)
+    ds = ctx.build_scene(s["positions"], s["triangles"])
+    assert ds.wide_nodes() > 0
+    n = [30001, 70001]
+    host = [entering_rays(s["positions"], s["triangles"], k, k) for k in n]
+    want = [(cuda.trace_closest(ctx, ds, r), cuda.trace_any(ctx, ds, r)) for r in host]
+    dev = [{k: torch.from_numpy(v).cuda() for k, v in r.items()} for r in host]
+    calls = 2 * streams + 9
+    outs = [({k: torch.empty(n[i % 2], dtype=torch.int32 if k == "slot" else torch.float32, device="cuda")
+              for k in ("slot", "t", "u", "v")}, torch.empty(n[i % 2], dtype=torch.uint8, device="cuda"))
+            for i in range(calls)]
+    queue = [torch.cuda.Stream() for _ in range(streams)]
+    torch.cuda.synchronize()
+    ctx.set_async_walker_share(share)
+    for i, (o, occ) in enumerate(outs):
+        cuda.trace_closest_device_async(ctx, ds, dev[i % 2], o, queue[i % streams].cuda_stream)
+        cuda.trace_any_device_async(ctx, ds, dev[i % 2], occ, queue[i % streams].cuda_stream)
+    torch.cuda.synchronize()
+    ctx.set_async_walker_share(50)
+    for i, (o, occ) in enumerate(outs):
+        same(({k: v.cpu().numpy() for k, v in o.items()}, occ.cpu().numpy()), want[i % 2])
+    assert ctx.device_error_bits() == 0
+    ds.close()
