@@ -607,9 +607,10 @@ static gpugi_status trace_host_async(gpugi_ctx* ctx, const gpugi_scene* sc, bool
     uint8_t* dOcc = reinterpret_cast<uint8_t*>(base + 7 * col);
     st = launch_trace_filtered_on(ctx, sc, anyHit, d[0], d[1], d[2], d[3], d[4], d[5], d[6], n,
                                   anyHit ? nullptr : dSlot, anyHit ? nullptr : dT, anyHit ? nullptr : dU,
-                                  anyHit ? nullptr : dV, anyHit ? dOcc : nullptr, ss->queue, ss->counters, s);
-    // (the full walker grid: host-array queries are paced by their copies,
-    // and a shorter walk keeps each stream's copy-trace-copy cycle short)
+                                  anyHit ? nullptr : dV, anyHit ? dOcc : nullptr, ss->queue, ss->counters, s, 100, 1,
+                                  n >= (1ull << 20) && streams_in_use(ctx) >= 3);
+    // (the full walker grid: host-array queries are paced by their copies, and a shorter walk keeps each
+    // stream's copy-trace-copy cycle short; long batches on several streams: launch_trace_filtered_on)
     if (st) return st;
     if ((st = copy_results_out(ctx, anyHit, dRes, 0, slot, t, u, v, occ, 0, n, s))) return st;
     GPUGI_CUDA_TRY(ctx, cudaEventRecord(ss->lastUse, s));

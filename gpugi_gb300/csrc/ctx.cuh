@@ -185,7 +185,7 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
                                       const float* dz, const float* tmax, uint64_t n, int32_t* slot, float* t,
                                       float* u, float* v, uint8_t* occluded, uint32_t* queue,
                                       unsigned long long* counters, cudaStream_t stream = nullptr,
-                                      uint32_t walkerShare = 100, uint32_t streams = 1);
+                                      uint32_t walkerShare = 100, uint32_t streams = 1, bool paced = false);
 // Launch shape of a persistent walker: grid, dynamic shared memory and the
 // number of top-of-tree nodes it stages (at most maxStage).
 struct WalkerLaunch {

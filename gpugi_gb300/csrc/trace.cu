@@ -352,17 +352,25 @@ __global__ void __launch_bounds__(128, GPUGI_GROUP_MIN_BLOCKS) k_trace_group(
 }
 
 // Second launch after the root prefilter on scenes with a wide hierarchy: one
-// lane walks each queued ray over it (wide_walks).
+// lane walks each queued ray over it (wide_walks). least > 0: only as many
+// blocks as give each warp kPacedRays rays, at least that many.
+constexpr uint32_t kPacedRays = 48;
 template <bool ANY_HIT, int TRI>
 __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide(
     DevScene s, const float* __restrict__ ox, const float* __restrict__ oy, const float* __restrict__ oz,
     const float* __restrict__ dx, const float* __restrict__ dy, const float* __restrict__ dz,
     const float* __restrict__ tmax, int32_t* __restrict__ slot, float* __restrict__ t, float* __restrict__ u,
     float* __restrict__ v, uint8_t* __restrict__ occluded, const uint32_t* __restrict__ queue,
-    unsigned long long* counters, uint32_t* err) {
+    unsigned long long* counters, uint32_t* err, uint32_t least) {
     __shared__ WideShared sh;
+    const uint64_t n = counters[1];
+    unsigned blocks = gridDim.x;
+    if (least) {
+        blocks = (unsigned)min((uint64_t)blocks, max((uint64_t)least, (n + 4 * kPacedRays - 1) / (4 * kPacedRays)));
+        if (blockIdx.x >= blocks) return;
+    }
     wide_walks<ANY_HIT, TRI>(
-        sh, s, counters[1], counters + 2, err,
+        sh, s, n, counters + 2, err,
         [&](uint64_t i, float3& o, float3& d, float& len) {
             const uint32_t ray = __ldg(queue + i);
             o = make_float3(__ldg(ox + ray), __ldg(oy + ray), __ldg(oz + ray));
@@ -379,7 +387,8 @@ __global__ void __launch_bounds__(128, GPUGI_WIDE_MIN_BLOCKS) k_trace_wide(
                 u[ray] = hitU;
                 v[ray] = hitV;
             }
-        });
+        },
+        blocks);
 }
 
 // At most kDirectRays rays per warp of the full grid, on scenes with a wide
@@ -476,13 +485,14 @@ gpugi_status launch_trace_filtered(gpugi_ctx* ctx, const gpugi_scene* sc, bool a
 
 // The same launches as launch_trace_filtered, on scratch memory the caller
 // provides (queue of n entries, 4 counters, which it zeroes on the stream);
-// allocates nothing. streams: how many the caller's queries are spread over.
+// allocates nothing. streams: how many the caller's queries are spread over;
+// paced: the batch lies between copies that take longer than its walk.
 gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, bool anyHit, const float* ox,
                                       const float* oy, const float* oz, const float* dx, const float* dy,
                                       const float* dz, const float* tmax, uint64_t n, int32_t* slot, float* t,
                                       float* u, float* v, uint8_t* occluded, uint32_t* queue,
                                       unsigned long long* counters, cudaStream_t stream, uint32_t walkerShare,
-                                      uint32_t streams) {
+                                      uint32_t streams, bool paced) {
     if (n == 0) return GPUGI_OK;
     cudaStream_t cs = stream ? stream : ctx->stream;
     const int ell = (int)sc->dev.boundsKind;  // bounds kind: 0 box, 1 ellipsoid, 2 oriented box
@@ -549,8 +559,16 @@ gpugi_status launch_trace_filtered_on(gpugi_ctx* ctx, const gpugi_scene* sc, boo
         //   8           59.5 / 54.5 / 53.1 / 52.7    66.0 / 61.8 / 61.7 / 63.6     836 / 837 / 839 / 888
         const uint32_t tenths = std::min(std::max(10u * streams, 28u), 56u);
         L.grid = std::max(1u, share_of_grid(L.grid, walkerShare) * 28u / tenths);
+        // Batches of 2^20 rays and more between copies over the host link, on three streams or more: a
+        // walk of a third of the time a batch's copies take makes copies of neighbouring streams meet in
+        // the link's directions, so short queues walk on part of the grid. Us a batch, whole grid / part,
+        // page-locked arrays, random rays at the 65k icosphere on 2 / 3 / 4 / 6 streams: 2^19 rays 111 / 136,
+        // 83 / 94, 82 / 89, 81 / 88; 3 x 2^18 156 / 180, 126 / 127, 125 / 125, 125 / 124; 2^20 198 / 218,
+        // 168 / 161, 168 / 161, 167 / 160; 2^21 353 / 361, 326 / 326, 326 / 326, 325 / 326. Long queues
+        // (aimed rays) have the whole grid on both sides.
+        const uint32_t least = paced ? std::max(1u, share_of_grid(L.grid, 28)) : 0u;
         kw<<<L.grid, 128, 0, cs>>>(sc->dev, ox, oy, oz, dx, dy, dz, tmax, slot, t, u, v, occluded, queue, counters,
-                                   ctx->errWord);
+                                   ctx->errWord, least);
         GPUGI_CUDA_TRY(ctx, cudaGetLastError());
         return GPUGI_OK;
     }

@@ -733,17 +733,18 @@ GPUGI_D void leaf_rounds(unsigned todo, const float4 (*ray)[128], const uint32_t
     }
 }
 
-// Persistent loop of wide walks over n work items in blocks of 128 threads:
-// the grid's warps share the first items out evenly (at most 32 each), later
-// ones come from an atomic counter *work, which starts at 0. load(i, o, d,
-// tmax) fills the ray of item i (again when a walk restarts); finish(i, slot,
-// t, u, v) takes its result (any hit: slot >= 0 when occluded). n < 2^32.
-// work may be null where every warp gets at most kWideSolo items: they are
-// then strided over the warps. MULTI: the items belong to several scenes, load returns the item's (a scene
-// with a wide hierarchy); otherwise every ray walks `scene`.
+// Persistent loop of wide walks over n work items in blocks of 128 threads, of
+// which the first `blocks` of the grid call it: their warps share the first
+// items out evenly (at most 32 each), later ones come from an atomic counter
+// *work, which starts at 0. load(i, o, d, tmax) fills the ray of item i (again
+// when a walk restarts); finish(i, slot, t, u, v) takes its result (any hit:
+// slot >= 0 when occluded). n < 2^32. work may be null where every warp gets at
+// most kWideSolo items: they are then strided over the warps. MULTI: the items
+// belong to several scenes, load returns the item's (a scene with a wide
+// hierarchy); otherwise every ray walks `scene`.
 template <bool ANY_HIT, int TRI, bool MULTI = false, typename Load, typename Finish>
 GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsigned long long* work, uint32_t* err, Load load,
-                        Finish finish) {
+                        Finish finish, unsigned blocks = gridDim.x) {
     constexpr uint32_t kNone = 0xFFFFFFFFu;  // also kWideEmpty: never a node or a leaf
     const unsigned lane = threadIdx.x & 31u;
     const DevScene* own = &scene;  // MULTI: the scene of the lane's ray
@@ -832,11 +833,11 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
         return (isinf(inv.x) && lo.x == o.x && hi.x == o.x) || (isinf(inv.y) && lo.y == o.y && hi.y == o.y) ||
                (isinf(inv.z) && lo.z == o.z && hi.z == o.z);
     };
-    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    const unsigned warps = blocks * (blockDim.x >> 5);
     const unsigned C = n >= 32 * (uint64_t)warps ? 32u : ((uint32_t)n + warps - 1) / warps;
     const uint64_t first = (uint64_t)warps * C;
     bool more = n > first;
-    const uint64_t warp = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint64_t warp = (uint64_t)(threadIdx.x >> 5) * blocks + blockIdx.x;
     const bool solo = n <= (uint64_t)warps * (ANY_HIT ? kWideSoloAny : kWideSolo);
     if (!solo) {
         const uint64_t i = warp * C + lane;

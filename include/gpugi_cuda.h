@@ -331,7 +331,8 @@ gpugi_status gpugi_set_host_pipeline(gpugi_ctx* ctx, uint32_t parts, uint32_t ze
  * last eight stream-ordered queries went to one or two streams; on more,
  * queries have 2.8 shares between them, down to half a share each.
  * Synchronous calls and host-array queries (paced by their copies) use the
- * full grid; results do not depend on the share. */
+ * full grid (batches of 2^20 rays and more on three streams and more walk
+ * short queues on part of it); results do not depend on the share. */
 gpugi_status gpugi_set_async_walker_share(gpugi_ctx* ctx, uint32_t percent);
 
 /* Scene layout tuning (set by the autotuner), applied to scenes uploaded

@@ -454,3 +454,44 @@ def test_shares_over_streams(ctx, streams, share):
         same(({k: v.cpu().numpy() for k, v in o.items()}, occ.cpu().numpy()), want[i % 2])
     assert ctx.device_error_bits() == 0
     ds.close()
+
+
+@pytest.mark.parametrize("streams", [2, 4])
+@pytest.mark.parametrize("entering", [0, 1, 5000, 70000, 400000])
+def test_long_host_batches_over_streams(ctx, streams, entering):
+    """2^20 + 1 rays in page-locked arrays of which 0 to 400,000 enter the scene: the walker's whole grid,
+    the least part of it and the part that the queue's length gives (three streams and more)."""
+    import ctypes
+
+    import torch
+    s = scenes.displaced_icosphere(16384, seed=4)
+    pos, tri = s["positions"], s["triangles"]
+    ds = ctx.build_scene(pos, tri)
+    n = (1 << 20) + 1
+    away = make_rays(np.full((n, 3), 10.0) * np.ptp(pos, axis=0).max(), np.full((n, 3), 3 ** -0.5), np.full(n, np.inf))
+    at = np.sort(np.random.default_rng(entering).permutation(n)[:entering])
+    rays = torch.empty((7, n)).pin_memory().numpy()
+    hit = entering_rays(pos, tri, max(1, entering), 3)
+    for k, key in enumerate(cuda.RAY_KEYS):
+        rays[k] = away[key]
+        rays[k, at] = hit[key][:entering]
+    want = cuda.trace_closest(ctx, ds, dict(zip(cuda.RAY_KEYS, rays)))
+    want_any = cuda.trace_any(ctx, ds, dict(zip(cuda.RAY_KEYS, rays)))
+    queue = [torch.cuda.Stream() for _ in range(streams)]
+    out = [torch.empty((4, n)).pin_memory().numpy() for _ in range(streams)]
+    occ = [torch.empty(n, dtype=torch.uint8).pin_memory().numpy() for _ in range(streams)]
+    lib, P = cuda.lib(), ctypes.c_void_p
+    lib.gpugi_trace_closest_async.argtypes = [P] * 9 + [ctypes.c_uint64] + [P] * 5
+    lib.gpugi_trace_any_async.argtypes = [P] * 9 + [ctypes.c_uint64] + [P] * 2
+    for _ in range(4):
+        for q, o, c in zip(queue, out, occ):
+            src = [r.ctypes.data for r in rays]
+            ctx.check(lib.gpugi_trace_closest_async(ctx.handle, ds.handle, *src, n, *[r.ctypes.data for r in o],
+                                                    q.cuda_stream))
+            ctx.check(lib.gpugi_trace_any_async(ctx.handle, ds.handle, *src, n, c.ctypes.data, q.cuda_stream))
+    torch.cuda.synchronize()
+    assert (want["slot"] >= 0).sum() >= 0.5 * entering
+    for o, c in zip(out, occ):
+        same((dict(zip(("slot", "t", "u", "v"), o)), c), (want, want_any))
+    assert ctx.device_error_bits() == 0
+    ds.close()
