@@ -852,6 +852,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
             base = first + __shfl_sync(0xffffffffu, base, 0);
             more = base + __popc(~act) < n;
             base += (unsigned)__popc(~act & ((1u << lane) - 1u));
+            __syncwarp();  // the leaf rounds' reads of the rays that are replaced
             if (!active && base < n) begin((uint32_t)base);
         } else if (!more && __popc(act) <= kWideWarpAt) {
             break;
@@ -960,6 +961,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
     // and resolves them in order.
     uint2* const ws = sh.w[threadIdx.x >> 5];
     uint64_t next = warp;
+    __syncwarp();  // a warp with few rays comes here straight from begin(), whose rays every lane reads
     while (true) {
         unsigned src = 0;
         if (solo) {
@@ -1227,6 +1229,7 @@ GPUGI_D void lane_walks(LaneShared& sh, const DevScene& s, uint64_t n, unsigned 
             base = first + __shfl_sync(0xffffffffu, base, 0);
             more = base + __popc(~act) < n;
             base += (unsigned)__popc(~act & ((1u << lane) - 1u));
+            __syncwarp();  // the leaf rounds' reads of the rays that are replaced
             if (!active && base < n) begin((uint32_t)base);
         } else if (!more && __popc(act) <= kLaneGroupAt) {
             break;
