@@ -25,7 +25,9 @@ struct gpugi_ctx {
     void* bounce = nullptr;
     void* bounceDev = nullptr;  // its device address
     // trace tuning
-    uint32_t traceMode = 3;  // 0 thread per ray, 1 persistent lane refill, 2 root prefilter + 1, 3 + wide walk or 8-lane groups, 4/5 + 4/16-lane groups
+    // 0 thread per ray, 1 persistent lane refill, 2 root prefilter + 1, 3 + wide walk, lane walk or 8-lane
+    // groups, 4/5 + 4/16-lane groups
+    uint32_t traceMode = 3;
     uint32_t traceBlock = 128;
     // photon mapper (PhotonMapper's pm_nphotons, pm_r, pm_progressive; photonmapper.cpp:17-45)
     uint32_t pmPhotonsPerSample = 1u << 11;

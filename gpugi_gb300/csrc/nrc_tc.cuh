@@ -62,10 +62,10 @@ GPUGI_D uint64_t globaltimer_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// Wait for the phase `parity` of an mbarrier, at most limitNs nanoseconds
-// of the global timer (and at most 2^24 polls, should the timer not
-// advance); false when the wait ran out. The timer is first read after 256
-// polls: a wait that ends sooner (every one but a lost one) never reads it.
+// Wait for the phase `parity` of an mbarrier; false when the wait ran out:
+// limitNs nanoseconds of the global timer after its 256th poll, looked at every
+// 256 polls, and at most 2^24 polls, should the timer not advance. A wait that
+// ends within 256 polls (every one but a lost one) never reads the timer.
 GPUGI_D bool bar_wait(uint64_t* bar, uint32_t parity, uint64_t limitNs) {
     const uint32_t a = smem_addr(bar);
     uint64_t t0 = 0;

@@ -31,8 +31,9 @@
 #include "shade.cuh"
 #include "trace.cuh"
 
-// On scenes without a wide hierarchy the passes' walkers walk a queue with
-// 8-lane groups while it holds fewer rays than this many times the resident lanes, and a ray per lane otherwise.
+// On scenes without a wide hierarchy whose top nodes are staged, the passes'
+// walkers walk a queue with 8-lane groups while it holds fewer rays than this
+// many times the resident lanes, and a ray per lane otherwise (group_below).
 #ifndef GPUGI_GROUP_BELOW_LANES
 #define GPUGI_GROUP_BELOW_LANES 2u
 #endif
@@ -530,8 +531,8 @@ GPUGI_D void pt_shade_lane(const RenderConst& rc, const PathSoA& A, const HitSoA
     L.survive = roulette(rc, depth, thr, L.tp, L.seed) && depth + 1 < rc.maxPathLength;
 }
 
-__global__ void __launch_bounds__(128, kShadeBlocks) k_pt_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q,
-                                                  int depth) {
+__global__ void __launch_bounds__(128, kShadeBlocks) k_pt_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H,
+                                                                ShadowSoA Q, int depth) {
     const uint32_t n = rc.cnt->path[depth];
     WARP_LOOP(n, k, valid) {
         PtLane L;
@@ -631,8 +632,8 @@ GPUGI_D void light_shade_lane(const RenderConst& rc, const PathSoA& A, const Hit
     L.o = L.o + L.d * kRAY_HIT_EPSILON;
 }
 
-__global__ void __launch_bounds__(128, kShadeBlocks) k_light_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H, ShadowSoA Q,
-                                                     int depth, bool withCache) {
+__global__ void __launch_bounds__(128, kShadeBlocks) k_light_shade(RenderConst rc, PathSoA A, PathSoA B, HitSoA H,
+                                                                   ShadowSoA Q, int depth, bool withCache) {
     const uint32_t n = rc.cnt->path[depth];
     WARP_LOOP(n, k, valid) {
         LightLane L;

@@ -1,4 +1,13 @@
-// Stackless escape-pointer BVH walk and its intersection tests (device code).
+// Ray walks over the scene's hierarchy and their intersection tests (device
+// code). All return trace_ray's results bit for bit:
+//   trace_ray     one thread per ray, stackless (escape pointers): the
+//                 reference's walk, which the others are held against
+//   walk_step     the same one test at a time, for warps that refill lanes
+//   group_walks   4, 8 or 16 lanes walk one ray together, stackless
+//   wide_walks    a depth-first stack over the four-wide copy of a box
+//                 hierarchy (wide.cu), a lane or a warp per ray
+//   lane_walks    the escape walk with leaves tested by eight lanes each, for
+//                 hierarchies without that copy
 //
 // Same walk as gpugi's TraceRay/TraceRayAnyHit (gpugi/shader/traceray.glsl:
 // 25-180): nodes are visited in preorder; a node whose bounds are hit with
@@ -743,13 +752,12 @@ GPUGI_D void leaf_rounds(unsigned todo, const float4 (*ray)[128], const uint32_t
 // belong to several scenes, load returns the item's (a scene with a wide
 // hierarchy); otherwise every ray walks `scene`.
 template <bool ANY_HIT, int TRI, bool MULTI = false, typename Load, typename Finish>
-GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsigned long long* work, uint32_t* err, Load load,
-                        Finish finish, unsigned blocks = gridDim.x) {
+GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsigned long long* work, uint32_t* err,
+                        Load load, Finish finish, unsigned blocks = gridDim.x) {
     constexpr uint32_t kNone = 0xFFFFFFFFu;  // also kWideEmpty: never a node or a leaf
     const unsigned lane = threadIdx.x & 31u;
     const DevScene* own = &scene;  // MULTI: the scene of the lane's ray
     const char* wide = reinterpret_cast<const char*>(scene.wide);
-    auto tris_of = [](const DevScene& s) { return TRI ? s.wtris : s.tris; };
     auto shfl_scene = [&](unsigned mask, unsigned src) {
         const uint64_t p = reinterpret_cast<uint64_t>(own);
         return reinterpret_cast<const DevScene*>((uint64_t)__shfl_sync(mask, (uint32_t)(p >> 32), src) << 32 |
@@ -866,10 +874,13 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     const uint32_t ax = at + (ivx.x < 0.0f ? 16u : 0u), ay = at + (ivy.x < 0.0f ? 48u : 32u),
                                    az = at + (ivz.x < 0.0f ? 80u : 64u);
                     auto ld = [&](uint32_t off) { return __ldg(reinterpret_cast<const float4*>(wide + off)); };
-                    const float4 nx = ld(ax), fx = ld(ax ^ 16u), ny = ld(ay), fy = ld(ay ^ 16u), nz = ld(az), fz = ld(az ^ 16u);
+                    const float4 nx = ld(ax), fx = ld(ax ^ 16u), ny = ld(ay), fy = ld(ay ^ 16u), nz = ld(az),
+                                 fz = ld(az ^ 16u);
                     const uint4 rf = __ldg(reinterpret_cast<const uint4*>(wide + (at + 96u)));
                     // slab values of two children's planes
-                    auto slab = [](float p, float q, float2 no, float2 iv) { return __fmul2_rn(__fadd2_rn(make_float2(p, q), no), iv); };
+                    auto slab = [](float p, float q, float2 no, float2 iv) {
+                        return __fmul2_rn(__fadd2_rn(make_float2(p, q), no), iv);
+                    };
                     const float2 nx0 = slab(nx.x, nx.y, nox, ivx), nx1 = slab(nx.z, nx.w, nox, ivx);
                     const float2 ny0 = slab(ny.x, ny.y, noy, ivy), ny1 = slab(ny.z, ny.w, noy, ivy);
                     const float2 nz0 = slab(nz.x, nz.y, noz, ivz), nz1 = slab(nz.z, nz.w, noz, ivz);
@@ -877,8 +888,10 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     const float2 fy0 = slab(fy.x, fy.y, noy, ivy), fy1 = slab(fy.z, fy.w, noy, ivy);
                     const float2 fz0 = slab(fz.x, fz.y, noz, ivz), fz1 = slab(fz.z, fz.w, noz, ivz);
                     auto widen = [](float l) { return TRI ? X::mul(l, 0x1.000008p+0f) : l; };
-                    const float f0 = fmaxf(0.0f, max3f(nx0.x, ny0.x, nz0.x)), f1 = fmaxf(0.0f, max3f(nx0.y, ny0.y, nz0.y));
-                    const float f2 = fmaxf(0.0f, max3f(nx1.x, ny1.x, nz1.x)), f3 = fmaxf(0.0f, max3f(nx1.y, ny1.y, nz1.y));
+                    const float f0 = fmaxf(0.0f, max3f(nx0.x, ny0.x, nz0.x));
+                    const float f1 = fmaxf(0.0f, max3f(nx0.y, ny0.y, nz0.y));
+                    const float f2 = fmaxf(0.0f, max3f(nx1.x, ny1.x, nz1.x));
+                    const float f3 = fmaxf(0.0f, max3f(nx1.y, ny1.y, nz1.y));
                     bool h0 = f0 <= widen(min3f(fx0.x, fy0.x, fz0.x)) && f0 <= len;
                     bool h1 = f1 <= widen(min3f(fx0.y, fy0.y, fz0.y)) && f1 <= len;
                     bool h2 = f2 <= widen(min3f(fx1.x, fy1.x, fz1.x)) && f2 <= len && rf.z != kWideEmpty;

@@ -2,14 +2,15 @@
 // the scene at hand (CUDA events on the context stream).
 //
 //  * ray queries: trace mode (thread per ray with block size 64/128/256,
-//    persistent lane refill, root prefilter + persistent walker) on
-//    synthetic rays over the scene's bounds;
+//    persistent lane refill, root prefilter + persistent walker, the default
+//    mode's walkers, 4- and 16-lane groups) on synthetic rays over the scene's
+//    bounds;
 //  * batched rendering: the path-queue capacity of a round (small rounds keep
 //    the wavefront state in L2, large rounds have fewer launches and
 //    shorter tails) on a 512 x 512 path-tracing job of the scene.
 //
-// The traversal is stackless (escape pointers), so there is no stack depth
-// to tune.
+// There is no stack depth to tune: the escape walks have none, and the wide
+// walk's is sized for every tree that it accepts.
 #include <algorithm>
 #include <cmath>
 #include <vector>

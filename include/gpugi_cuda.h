@@ -274,11 +274,12 @@ gpugi_status gpugi_trace_any_async(gpugi_ctx* ctx, const gpugi_scene* scene,
  * (cudaGetSymbolAddress); make that first call before any stream capture.
  * All calls share the one array: calls that overlap on the GPU (other
  * streams, other contexts on the same device) race and must be serialised
- * by the caller. Asynchronous on the context stream. It always runs the
- * root prefilter and a queue walker (trace mode 2 when the context is set to
- * mode 0, 1 or 2, the context's walker for modes 3-5): modes 0 and 1
- * need no queue and have no allocation-free form, and every mode returns the
- * same results. */
+ * by the caller. Asynchronous on the context stream. It runs the root
+ * prefilter and a queue walker (trace mode 2 when the context is set to mode
+ * 0, 1 or 2, the context's walker for modes 3-5; small calls in mode 3 as
+ * gpugi_set_trace_config says, which leaves the array untouched): modes 0 and
+ * 1 need no queue and have no allocation-free form, and every mode returns
+ * the same results. */
 #define GPUGI_NOALLOC_MAX_RAYS (1u << 20)
 gpugi_status gpugi_trace_closest_noalloc(gpugi_ctx* ctx, const gpugi_scene* scene,
                                          const float* ox, const float* oy, const float* oz,
@@ -300,15 +301,21 @@ gpugi_status gpugi_trace_stats_device(gpugi_ctx* ctx, const gpugi_scene* scene,
  * finished lanes from a device ray counter; mode 2: a coalesced
  * root-bounds prefilter that finishes rays missing the scene and queues the
  * rest (warp-ballot compaction) for the persistent walker; mode 3
- * (default): the same prefilter, then, on box hierarchies whose boxes nest
- * (every one that bvhmake or gpugi_scene_build makes), a walk over a four-wide
- * copy of the hierarchy, one lane per ray with leaves tested by eight lanes,
- * and on other scenes a walk of the hierarchy itself, one lane per ray for long
- * queues and for short ones groups of 8 lanes that walk one ray together,
- * testing a window of consecutive preorder nodes or leaf slots per round;
- * modes 4 and 5: such groups of 4 and 16 lanes on every scene. All modes make the same
- * decisions per ray as TraceRay and return identical results. blockSize
- * applies to mode 0. */
+ * (default): the same prefilter, then, on scenes with a four-wide copy of
+ * their hierarchy, a walk over that, one lane per ray with leaves tested by
+ * eight lanes (a warp per ray for short queues; calls of at most two rays per
+ * warp of the full grid, 9,728 on 152 SMs, take one launch without prefilter
+ * and queue), and on other scenes a walk of the hierarchy itself, one lane per
+ * ray for long queues and for short ones groups of 8 lanes that walk one ray
+ * together, testing a window of consecutive preorder nodes or leaf slots per
+ * round; modes 4 and 5: such groups of 4 and 16 lanes on every scene. All
+ * modes make the same decisions per ray as TraceRay and return identical
+ * results. blockSize applies to mode 0.
+ * Upload and build make the four-wide copy of box hierarchies of at least
+ * three nodes that are preorder trees with two children per inner node and
+ * whose boxes nest (what bvhmake and gpugi_scene_build write), unless staged
+ * top nodes were asked for (gpugi_set_scene_layout), the tree has more than 24
+ * four-wide levels or 2^25 four-wide nodes, or memory for the copy is lacking. */
 gpugi_status gpugi_set_trace_config(gpugi_ctx* ctx, uint32_t mode, uint32_t blockSize);
 
 /* Host-pointer ray queries (gpugi_trace_closest / gpugi_trace_any). The
@@ -494,7 +501,7 @@ gpugi_status gpugi_nrc_set_weights(gpugi_ctx* ctx, gpugi_nrc* nrc, const float* 
 #define GPUGI_NRC_KERNELS_MMA_SYNC 1u
 gpugi_status gpugi_nrc_set_kernels(gpugi_ctx* ctx, gpugi_nrc* nrc, uint32_t kernels);
 /* Every mbarrier wait of the tcgen05 kernels is bounded (1 s of the global
- * timer by default); a wait that runs out sets GPUGI_DEVERR_WAIT_TIMEOUT, the
+ * timer by default, from the wait's 256th poll on); a wait that runs out sets GPUGI_DEVERR_WAIT_TIMEOUT, the
  * kernel frees its tensor memory and ends, and the context stays usable.
  * Test support: with stall = 1 those kernels issue no MMA and no commit, so
  * their first wait runs out after waitNs nanoseconds (0 = the default 1 s);
@@ -669,8 +676,8 @@ gpugi_status gpugi_measure_l2_bandwidth(gpugi_ctx* ctx, uint64_t bytes, uint32_t
  * GPUGI_TUNE_TRACE: ray-query kernels (gpugi_set_trace_config mode and block
  * size) on 2^20 synthetic rays over the scene bounds; GPUGI_TUNE_BATCH: the
  * path-queue capacity of batched rounds on a 512 x 512, 64-spp PT job
- * (needs vertex info and materials). The traversal is stackless, so no stack
- * depth is tuned. Synchronises; allocates temporary buffers. */
+ * (needs vertex info and materials). The walks have no stack depth to tune.
+ * Synchronises; allocates temporary buffers. */
 #define GPUGI_TUNE_TRACE 1u
 #define GPUGI_TUNE_BATCH 2u
 typedef struct gpugi_tuning {
