@@ -623,12 +623,12 @@ GPUGI_D void group_walks_multi(uint64_t n, unsigned long long* work, uint32_t* e
 //    the binary tree at once. (The watertight box test drops those slabs on
 //    every level, so it stays monotone.)
 //
-// What bounds it and why this split (98k-triangle room, 4.2M rays a launch,
-// ncu): L1 wavefronts 82 % busy and issue slots 70 %, DRAM idle: a lane reads
-// 112 B of node per visit, 10 visits per ray instead of 45 binary nodes. One
-// lane per ray for nodes keeps an instruction useful for ~20 lanes (8-lane
-// groups on 8-wide nodes issued 2.3x the instructions); leaves go to eight
-// lanes each, four leaves at a time, because a lane that loops over a block's
+// What bounds it and why this split (98k-triangle room, second bounce of 4.2M
+// camera paths, ncu): L1 wavefronts 83 % and issue slots 71 % of their peaks,
+// DRAM 1 % (camera rays 58 % and 78 %): a lane reads 112 B of node per visit, 10
+// visits per ray instead of 45 binary nodes. One lane per ray for nodes keeps
+// an instruction useful for ~20 lanes (8-lane groups on 8-wide nodes issued 2.3x
+// the instructions); leaves go to eight lanes each, four leaves at a time, because a lane that loops over a block's
 // triangles waits for memory once per triangle (1.05 to 0.87 ms for 3M
 // any-hit rays in the 528k-triangle terrain, then). Quantised 96-B nodes halved
 // the L1 load but cost more issue slots than they freed (0.99 ms); prefetches
