@@ -1017,12 +1017,9 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
             __syncwarp();
         }
         // `leaves` leading leaves, lane group g's word lref with entry distance lf; true when any hit is
-        // done. A leaf is entered once, with the rayLength of that moment: a block of several passes of
-        // eight lanes (always alone) is not tested against its own hits, which rounding can place before
-        // its box. Leaves that are tested together take one pass each and are entered in order below.
+        // done. Leaves that are tested together take one pass of eight lanes each.
         auto test_leaves = [&](uint32_t lref, float lf, unsigned leaves) {
             const unsigned g = lane >> 3, gl = lane & 7u;
-            const bool enter = lf <= wlen;
             const uint32_t k0 = g < leaves ? (lref & LEAF_BLOCK_MASK) * s.leafSize : 0u;
             const uint32_t cnt = g < leaves ? leaf_slots(s, lref, err) : 0u;
             for (uint32_t off = gl; __any_sync(0xffffffffu, off - gl < cnt); off += 8) {
@@ -1033,7 +1030,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
                     ok = TRI ? intersect_triangle_wt_v(o, wt, a, b, c, h, hu, hv)
                              : intersect_triangle_v(o, d, a, b, c, h, hu, hv);
-                    ok = ok && enter && h < wlen;
+                    ok = ok && h < wlen && lf <= wlen;
                 }
                 if (!__any_sync(0xffffffffu, ok)) continue;
                 if (ANY_HIT) {
@@ -1050,7 +1047,7 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                     if (!gm) continue;
                     const unsigned win = 8 * k + (unsigned)__ffs(gm) - 1;
                     const float kf = __shfl_sync(0xffffffffu, lf, win), kh = __shfl_sync(0xffffffffu, h, win);
-                    if ((leaves == 1 || kf <= wlen) && kh < wlen) {
+                    if (kf <= wlen && kh < wlen) {
                         wlen = kh;
                         wu = __shfl_sync(0xffffffffu, hu, win);
                         wv = __shfl_sync(0xffffffffu, hv, win);
@@ -1090,10 +1087,17 @@ GPUGI_D void wide_walks(WideShared& sh, const DevScene& scene, uint64_t n, unsig
                 const bool leaf = (e.x & LEAF_FLAG) != 0, large = (e.x >> LEAF_COUNT_SHIFT & LEAF_COUNT_MASK) > 8;
                 const unsigned lm = __ballot_sync(0xffffffffu, leaf);
                 // leading leaves; one at a time where a block takes more than one pass of eight lanes
-                const unsigned lead = __any_sync(0xffffffffu, leaf && large) ? 1u
-                                      : lm == 0xffffffffu ? 4u : ((unsigned)__ffs(~lm) - 1) / 8;
+                const bool several = __any_sync(0xffffffffu, leaf && large);
+                const unsigned lead = several ? 1u : lm == 0xffffffffu ? 4u : ((unsigned)__ffs(~lm) - 1) / 8;
                 wsp -= lead;
-                if (test_leaves(e.x, __uint_as_float(e.y), lead)) break;
+                float lf = __uint_as_float(e.y);
+                if (several) {
+                    // a leaf is entered once: not compared again with the rayLength that its own earlier
+                    // passes left, which rounding can put before its box
+                    if (!(__shfl_sync(0xffffffffu, lf, 0) <= wlen)) continue;
+                    lf = 0.0f;
+                }
+                if (test_leaves(e.x, lf, lead)) break;
                 continue;
             }
             if (wbudget == 0) {
